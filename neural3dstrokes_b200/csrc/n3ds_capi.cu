@@ -125,10 +125,8 @@ Resolved resolve(const n3ds_options_t* o) {
   r.warps = o->warps > 0 ? o->warps : 16;
   r.schedule = o->schedule == N3DS_SCHEDULE_RUNS ? N3DS_SCHEDULE_RUNS : N3DS_SCHEDULE_SEGMENTS;
   const bool runs = r.schedule == N3DS_SCHEDULE_RUNS;
-  // 24 warps only for the forward segment kernel (76 registers); the others hold
-  // 100+ registers per thread and run at most 16
-  // instantiated CTA sizes: segment forward 4-32 warps (64 registers), segment backward
-  // 4-24 (94 registers at 20 warps, 80 with a small spill at 24), run kernels 4-16
+  // instantiated CTA sizes: segment kernels 4-32 warps (64 registers at 32), run
+  // kernels (100+ registers) 4-16
   // largest instantiated CTA size not above the request
   auto pick = [](int w, std::initializer_list<int> sizes) {
     int best = 4;
@@ -136,11 +134,14 @@ Resolved resolve(const n3ds_options_t* o) {
       if (s <= w && s > best) best = s;
     return best;
   };
-  // defaults: the fastest measured on the benchmark workloads (32 / 24 for segments)
+  // defaults: the fastest measured on the benchmark workloads. Segment backward: 28 warps
+  // (72 registers, 16 bytes of spill), seven per scheduler against the exposed latency of
+  // record loads and shuffles; 32 would spill 60 bytes in the stroke loop (16 uneven
+  // mixed scenes: 24 warps 4.34 ms, 28 4.16, 32 4.48; 2000 curves 1.73 / 1.75 / 1.76)
   const int wf = o->warps > 0 ? o->warps : (runs ? 16 : 32);
-  const int wb = o->warps_bwd > 0 ? o->warps_bwd : (runs ? 16 : 24);
+  const int wb = o->warps_bwd > 0 ? o->warps_bwd : (runs ? 16 : 28);
   r.warps_fwd = runs ? pick(wf, {4, 8, 16}) : pick(wf, {4, 8, 16, 24, 32});
-  r.warps_bwd = runs ? pick(wb, {4, 8, 16}) : pick(wb, {4, 8, 16, 20, 24, 32});
+  r.warps_bwd = runs ? pick(wb, {4, 8, 16}) : pick(wb, {4, 8, 16, 20, 24, 28, 32});
   r.warps = r.warps_bwd;
   const size_t budget = size_t(di.smem_optin) - 256;  // room for static shared memory
   // default stages: the largest multiple of 32 strokes that fits the shared memory

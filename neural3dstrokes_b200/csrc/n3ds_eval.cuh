@@ -82,10 +82,10 @@ __device__ __forceinline__ float pair_alpha_common(const float* rec, V3 x, float
 
 // dL/dm of the soft step given G = (1 - alpha) dL/dalpha (division-safe form).
 __device__ __forceinline__ float soft_dm_from_G(int mode, float m, float alpha, float G) {
-  if (mode == STEP_LAPLACE) return m <= 0.f ? G * alpha / (1.f - alpha) : G;
+  if (mode == STEP_LAPLACE) return m <= 0.f ? __fdividef(G * alpha, 1.f - alpha) : G;
   if (mode == STEP_LINEAR) {
     float a = m + 0.5f;
-    return (a > 0.f && a < 0.9999f) ? G / (1.f - alpha) : 0.f;
+    return (a > 0.f && a < 0.9999f) ? __fdividef(G, 1.f - alpha) : 0.f;
   }
   return 0.f;
 }
@@ -106,18 +106,18 @@ __device__ __forceinline__ float soft_dm(int mode, float m, float alpha, float g
 // compat != 0: the reference formulas (no scale/position dependence through the
 // soft-step width, cube exterior 2*max(q,0)).
 __device__ __forceinline__ V3 prim_backprop(const float* rec, int kind, V3 p, float dsdf, float K,
-                                            float* v, int compat) {
+                                            float* v, int compat, V3 gsdf, const float* gbp) {
   int base = kind & 15;
   int flags = (kind >> 4) & 15;
-  float gbp[2];
-  V3 gp = prim_grad(base, p, rec, gbp, compat) * dsdf;
+  V3 gp = gsdf * dsdf;
   v[G_BP] += gbp[0] * dsdf;
   v[G_BP2] += gbp[1] * dsdf;
-  V3 s = xyz(rec4(rec)[R_S / 4]), si = xyz(rec4(rec)[R_SINV / 4]);
-  V3 q = s * p;
+  const V3 si = xyz(rec4(rec)[R_SINV / 4]);
   float kfac = compat ? 0.f : K;
   if ((kind & K_S3FAC) && !compat) {
+    const V3 s = xyz(rec4(rec)[R_S / 4]);
     if (base == B_SPHERE) {
+      const V3 q = s * p;
       // f = |q|/|p|: dL/dp += K (s^2 p/|q|^2 - p/|p|^2); dL/ds_i += K p_i^2 s_i/|q|^2
       float pp = dot(p, p), qq = dot(q, q);
       gp += (s * q) * (K / qq) + p * (-K / pp);
@@ -151,7 +151,8 @@ __device__ __forceinline__ V3 prim_backprop(const float* rec, int kind, V3 p, fl
     v[G_SCALE + 2] += -gp.z * p.z * si.z;
   }
   if (flags & F_R) {
-    V3 tq = cross(gp * si, q);
+    // (S^-1 g_p) x (S p); one scale cancels
+    const V3 tq = (flags & F_S3) ? cross(gp * si, xyz(rec4(rec)[R_S / 4]) * p) : cross(gp, p);
     v[G_TORQUE + 0] += tq.x;
     v[G_TORQUE + 1] += tq.y;
     v[G_TORQUE + 2] += tq.z;
@@ -161,6 +162,13 @@ __device__ __forceinline__ V3 prim_backprop(const float* rec, int kind, V3 p, fl
   v[G_GP + 2] += gp.z;
   // dL/dx = M^T gp
   return xyz(rec4(rec)[R_M / 4]) * gp.x + xyz(rec4(rec)[R_M / 4 + 1]) * gp.y + xyz(rec4(rec)[R_M / 4 + 2]) * gp.z;
+}
+
+__device__ __forceinline__ V3 prim_backprop(const float* rec, int kind, V3 p, float dsdf, float K,
+                                            float* v, int compat) {
+  float gbp[2];
+  const V3 g = prim_grad(kind & 15, p, rec, gbp, compat);
+  return prim_backprop(rec, kind, p, dsdf, K, v, compat, g, gbp);
 }
 
 // Warp transpose-reduction of NV per-lane values: after it, lane l holds the warp

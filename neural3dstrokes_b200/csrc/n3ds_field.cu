@@ -403,14 +403,20 @@ __device__ __forceinline__ void reduce_into(float (&v)[NV], float* row, int lane
 
 struct CompAdj {
   float T, Ps, Pr, Pg, Pb;          // running (through the previous stroke)
-  float gs, gcr, gcg, gcb, gT;      // seeds
-  float sig, Cr, Cg, Cb, Tf;        // forward totals
+  float gs, gcr, gcg, gcb;          // seeds
+  float sig, Cr, Cg, Cb;            // forward totals
+  float K;                          // exact: g_T T_final; compat: T_final
 };
 
 // Compose step + exact adjoint for one stroke; returns dL/dm. Writes colour /
-// density slots. compat: the reference compose adjoint (compositing.cu:104-155).
-__device__ __forceinline__ float compose_step(const float* rec, float a, float m, int mode, CompAdj& s,
-                                              float* v, int compat) {
+// density slots. The prefixes repeat the forward's accumulations bit for bit, so a
+// suffix (total minus prefix) carries rounding of the strokes below alone and is exactly
+// zero behind an opaque stroke. (One running scalar for the upstream-weighted suffix
+// takes 9 floats less, so 32 warps fit, 3.93 ms; but its rounding against the forward's
+// totals raised the softness gradient's error from 1.5e-6 to 2.2e-6 of its norm.)
+// compat: the reference compose adjoint (compositing.cu:104-155).
+template <int COMPAT>
+__device__ __forceinline__ float compose_step(const float* rec, float a, float m, int mode, CompAdj& s, float* v) {
   const float d = rec[R_DENSITY];
   const float4 col = rec4(rec)[R_COLOR / 4];
   const float c0 = col.x, c1 = col.y, c2 = col.z;
@@ -425,13 +431,13 @@ __device__ __forceinline__ float compose_step(const float* rec, float a, float m
   v[G_COLOR + 2] += s.gcb * w;
   v[G_DENSITY] += s.gs * w;
   float dm;
-  if (!compat) {
+  if (!COMPAT) {
     const float G = s.gs * (T1 * d - (s.sig - s.Ps)) + s.gcr * (T1 * c0 - (s.Cr - s.Pr)) +
-                    s.gcg * (T1 * c1 - (s.Cg - s.Pg)) + s.gcb * (T1 * c2 - (s.Cb - s.Pb)) - s.gT * s.Tf;
+                    s.gcg * (T1 * c1 - (s.Cg - s.Pg)) + s.gcb * (T1 * c2 - (s.Cb - s.Pb)) - s.K;
     dm = soft_dm_from_G(mode, m, a, G);
   } else {
     // reference: dL/da = [g_d (T' d - suf_d) + sum g_c O (T' c (O - a) - suf_c) / O^2] / max(1 - a, 1e-6)
-    const float O = 1.0f + 1e-6f - s.Tf;
+    const float O = 1.0f + 1e-6f - s.K;
     const float sc = 1.f / fmaxf(1.0f - a, 1e-6f);
     float ga = s.gs * (T1 * d - (s.sig - s.Ps)) * sc;
     ga += (s.gcr * (T1 * c0 * (O - a) - (s.Cr - s.Pr)) + s.gcg * (T1 * c1 * (O - a) - (s.Cg - s.Pg)) +
@@ -465,6 +471,11 @@ __device__ __forceinline__ void compose_skip(const float* rec, float a, CompAdj&
 // masks were recorded at another threshold (their tag), it visits every block: the
 // per-candidate test of the skip threshold makes the decisions culling would make.
 // STATS: count the evaluated pairs into L.stats (non-null).
+// Bound: issue slots, and the latency of record loads, shuffles and shared atomics (about
+// 300 warp instructions per segment and kept stroke, a fifth of them the 16-slot
+// reduction). 16 uneven mixed scenes, 347k rays x 64 samples: 4.77 ms at 24 warps; 4.34
+// with SDF and gradient in one type switch, the one scale cancelled in the torque, g_T
+// T_final formed once per segment and a fast division; 4.16 at 28 warps (72 registers).
 template <int WARPS, bool GX, int COMPAT, bool MASKS, bool STATS>
 __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_constant__ SegLaunch L) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -516,21 +527,22 @@ __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_con
           CompAdj s;
           {
             const float* st = L.state + 5 * c.si;
-            s.Tf = st[0]; s.sig = st[1]; s.Cr = st[2]; s.Cg = st[3]; s.Cb = st[4];
+            s.K = st[0]; s.sig = st[1]; s.Cr = st[2]; s.Cg = st[3]; s.Cb = st[4];
             const float* sd = L.seeds + 5 * c.si;
-            s.gs = sd[0]; s.gcr = sd[1]; s.gcg = sd[2]; s.gcb = sd[3]; s.gT = sd[4];
+            s.gs = sd[0]; s.gcr = sd[1]; s.gcg = sd[2]; s.gcb = sd[3];
+            if (!COMPAT) s.K *= sd[4];
             if (!c.active) {
-              s.gs = s.gcr = s.gcg = s.gcb = s.gT = 0.f;
+              s.gs = s.gcr = s.gcg = s.gcb = 0.f;
+              if (!COMPAT) s.K = 0.f;
             }
           }
-          V3 gx;
+          V3 gx = v3(0.f, 0.f, 0.f);
           if (sc.first_pass) {
             s.T = 1.f; s.Ps = s.Pr = s.Pg = s.Pb = 0.f;
-            gx = v3(0.f, 0.f, 0.f);
           } else {
             const float* b = L.bstate + 8 * c.si;
             s.T = b[0]; s.Ps = b[1]; s.Pr = b[2]; s.Pg = b[3]; s.Pb = b[4];
-            gx = GX ? v3(b[5], b[6], b[7]) : v3(0.f, 0.f, 0.f);
+            if (GX) gx = ld3(b + 5);
           }
           const unsigned nact = __popc(__ballot_sync(0xffffffffu, c.active));
           // The chunk's blocks (at most 32: stages hold at most 1024 strokes, in multiples
@@ -581,7 +593,9 @@ __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_con
     #pragma unroll
                 for (int j = 0; j < 16; j++) v[j] = -0.f;
                 const V3 p = prim_local(rec, c.x);
-                const float sdf = prim_sdf(base, p, rec);
+                V3 gsdf;
+                float gbp[2];
+                const float sdf = COMPAT ? prim_sdf(base, p, rec) : prim_sdf_grad(base, p, rec, &gsdf, gbp);
                 const float f = (kind & K_S3FAC) ? s3_factor(base, p, xyz(rec4(rec)[R_S / 4]), rec) : 1.f;
                 const float kk = h.y * f * c.rinv;
                 const float m = -sdf * kk;
@@ -591,10 +605,11 @@ __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_con
                   compose_skip(rec, a, s);
                   continue;
                 }
-                const float dm = compose_step(rec, a, m, mode, s, v, compat);
+                const float dm = compose_step<COMPAT>(rec, a, m, mode, s, v);
                 const float K = m * dm;
                 v[G_K] += K;
-                const V3 gp = prim_backprop(rec, kind, p, -kk * dm, K, v, compat);
+                const V3 gp = COMPAT ? prim_backprop(rec, kind, p, -kk * dm, K, v, compat)
+                                     : prim_backprop(rec, kind, p, -kk * dm, K, v, 0, gsdf, gbp);
                 if (GX) gx += gp;
                 reduce_into<16>(v, row, lane);
               } else if (base == B_QUAD_BEZIER) {
@@ -611,7 +626,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_con
                   compose_skip(rec, a, s);
                   continue;
                 }
-                const float dm = compose_step(rec, a, m, mode, s, v, compat);
+                const float dm = compose_step<COMPAT>(rec, a, m, mode, s, v);
                 v[G_K] += m * dm;
                 const V3 gq = quad_adjoint(rec, qf, -kk * dm, v + G_CTRL);
                 if (GX) gx += gq;
@@ -630,7 +645,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_con
                   compose_skip(rec, a, s);
                   continue;
                 }
-                const float dm = compose_step(rec, a, m, mode, s, v, compat);
+                const float dm = compose_step<COMPAT>(rec, a, m, mode, s, v);
                 const float dsdf = -kk * dm;
                 v[G_K] += m * dm;
                 V3 g = cubic_adjoint(rec, c.x, cf, dsdf, v + G_CTRL, compat, base == B_CATMULL_ROM);
@@ -1307,7 +1322,8 @@ cudaError_t launch_seg_bwd(const SegLaunch& L, int grid, int warps, size_t smem,
     case 16: return launch_bwd_w<16>(L, grid, smem, st);
     case 20: return launch_bwd_w<20>(L, grid, smem, st);
     case 24: return launch_bwd_w<24>(L, grid, smem, st);
-    case 32: return launch_bwd_w<32>(L, grid, smem, st);  // 64 registers, a small spill
+    case 28: return launch_bwd_w<28>(L, grid, smem, st);
+    case 32: return launch_bwd_w<32>(L, grid, smem, st);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -193,6 +193,54 @@ __device__ __forceinline__ V3 prim_grad(int base, V3 p, const float* rec, float*
   }
 }
 
+// prim_sdf and the exact prim_grad of the common primitives in one pass over the type
+// switch, sharing the folded coordinates (the other bases: two calls).
+__device__ __forceinline__ float prim_sdf_grad(int base, V3 p, const float* rec, V3* g, float* gbp) {
+  gbp[0] = 0.f;
+  gbp[1] = 0.f;
+  switch (base) {
+    case B_SPHERE: {
+      const float n2 = dot(p, p) + 1e-8f;
+      *g = p * rsqrtf(n2);
+      return sqrtf(n2) - 1.f;
+    }
+    case B_CUBE: {
+      const V3 q = sub1(vabs(p), 1.f), sg = vsgn(p), qp = vmax0(q);
+      const float n2 = dot(qp, qp), mx = max3(q);
+      *g = mx <= 0.f ? cube_inside_axis(q, sg) : sg * (qp * rsqrtf(n2));
+      return sqrtf(n2) + fminf(mx, 0.f);
+    }
+    case B_ROUND_CUBE: {
+      const V3 q = sub1(vabs(p), 1.f), sg = vsgn(p), qp = vmax0(q);
+      const float n2 = dot(qp, qp) + 1e-8f, mx = max3(q);
+      *g = sg * (qp * rsqrtf(n2));
+      if (mx < 0.f) *g += cube_inside_axis(q, sg);
+      gbp[0] = -1.f;
+      return sqrtf(n2) + fminf(mx, 0.f) - rec[R_BP];
+    }
+    case B_CAPSULE: {
+      const float bp = rec[R_BP], y = p.y;
+      p.y -= clampf(y, -bp, bp);
+      const float n2 = dot(p, p) + 1e-8f, inv = rsqrtf(n2);
+      gbp[0] = -sgn(y) * p.y * inv;
+      *g = p * inv;
+      return sqrtf(n2) - 1.f;
+    }
+    case B_OCTAHEDRON:
+      *g = vsgn(p) * OCTA_K;
+      return (fabsf(p.x) + fabsf(p.y) + fabsf(p.z) - 1.f) * OCTA_K;
+    case B_TETRAHEDRON: {
+      const float a = p.x + p.y, c = p.x - p.y, fa = fabsf(a) - p.z, fc = fabsf(c) + p.z;
+      const float sa = sgn(a) * OCTA_K, sc = sgn(c) * OCTA_K;
+      *g = fa > fc ? V3{sa, sa, -OCTA_K} : V3{sc, -sc, OCTA_K};
+      return (fmaxf(fa, fc) - 1.f) * OCTA_K;
+    }
+    default:
+      *g = prim_grad(base, p, rec, gbp, 0);
+      return prim_sdf(base, p, rec);
+  }
+}
+
 // Radius factor f of a multi-scale transform under inv_scale_radius
 // (strokes_forward.cu:74-81): f = |g*s| / |g| with g the SDF gradient direction.
 // For the sphere base g is parallel to p, so f = |s*p| / |p|.

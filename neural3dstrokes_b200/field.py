@@ -25,7 +25,7 @@ class FieldOptions:
     chunk_fwd: int = 0         # strokes per shared-memory stage (0: auto)
     chunk_bwd: int = 0
     warps: int = 0             # warps per CTA, forward: 4, 8, 16, 24, 32 (0: auto)
-    warps_bwd: int = 0         # warps per CTA, backward: 4, 8, 16, 20, 24 (0: auto)
+    warps_bwd: int = 0         # warps per CTA, backward: 4, 8, 16, 20, 24, 28, 32 (0: auto)
     schedule: str = "auto"     # 'segments' (auto): lane = sample; 'runs': packed (sample, stroke) pairs
     grad_mode: str = "exact"   # 'exact' or 'compat'
     forward_only: bool = False  # no backward follows: skip the bookkeeping the backward reads

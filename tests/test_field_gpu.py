@@ -266,3 +266,18 @@ def test_common_primitive_build_matches_general_build(cuda, kind):
     torch.autograd.backward([rgb, acc, depth], up)
     for ours, leaf in zip((f.grad_x, f.grad_shape, f.grad_color, f.grad_density, f.grad_delta), leaves):
         assert rel(ours, leaf.grad) < 1e-5
+
+
+@pytest.mark.parametrize("n_samples,opaque", [(1, False), (32, True), (33, False)])
+def test_multi_pass_backward_matches_float64(cuda, n_samples, opaque):
+    """The default 28-warp backward with its running composite state carried between
+    passes of one 32-stroke stage each, at segment edges."""
+    sc, rays = small_workload("mixed", n_strokes=70, n_rays=40, n_samples=n_samples, seed=17)
+    g = torch.Generator().manual_seed(9)
+    g_rgb, g_acc = torch.randn(rays.n_rays, 3, generator=g), torch.randn(rays.n_rays, generator=g)
+    (rgb, acc, _), leaves = run_field(sc, rays, cuda, opaque=opaque, requires_grad=True,
+                                      opts=FieldOptions(chunk_fwd=32, chunk_bwd=32))
+    torch.autograd.backward([rgb, acc], [g_rgb.to(cuda), g_acc.to(cuda)])
+    ref = oracle_grads(sc, rays, g_rgb, g_acc, torch.zeros(rays.n_rays), opaque=opaque)
+    for name, leaf in zip(("x", "shape", "color", "density", "delta"), leaves):
+        assert rel(leaf.grad, ref[name]) < GRAD_TOL, name
