@@ -120,6 +120,7 @@ _SIGS = {
                                                 _P, c_u32, c_i32, c_u32, c_i32, _P]),
     "n3ds_grid_encode_backward": (ctypes.c_int, [_P, _P, _P, _P, _P, c_u32, c_u32, c_u32, c_u32, ctypes.c_float,
                                                  c_u32, _P, _P, c_u32, c_i32, c_u32, c_i32, _P]),
+    "n3ds_grid_transpose": (ctypes.c_int, [_P, _P, c_u32, c_u32, c_u32, c_i32, _P]),
     "n3ds_grid_total_variation": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_float, c_u32, c_u32, c_u32, c_u32,
                                                  ctypes.c_float, c_u32, c_u32, c_i32, c_i32, _P]),
     "n3ds_density_net_feature_stride": (ctypes.c_int, [c_u32, c_u32]),

@@ -19,6 +19,7 @@
 //
 // Traffic per (point, level), C = 4 floats: 12 B input, 8 x 16 B corner rows (L2
 // hits once a level's table is resident), 16 B output; dy_dx adds D x 16 B.
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <type_traits>
@@ -292,6 +293,46 @@ __global__ void __launch_bounds__(kThreads) grid_tv_kernel(const T* __restrict__
   scatter_row<T, C>(grad + ((size_t)lv.base + row) * C, vec_table, v);
 }
 
+// [L, B] <-> [B, L] of units of U vectors V (a unit: the C channels of one point and
+// level), `tile` points per block through shared memory: the level-major side moves
+// tile * U vectors per level, the point-major side tile * L * U, both contiguous. The
+// encoder's kernels keep the level-major layout (a level's outputs or upstream gradients
+// are one stream while its table is in L2); its caller has one row of features per point.
+// HBM bound: 1,048,640 points x 10 levels x 16 B, 336 MB moved: 164 us as a strided copy,
+// 57 us here. (Kernels that read and write the rows directly lose more: half-
+// and whole-sector accesses 160 B apart took the forward from 258 to 346 / 320 us and the
+// backward from 452 to 541 / 560 us with one / two levels per thread.)
+template <typename V, int U, bool TO_ROWS>
+__global__ void __launch_bounds__(kThreads) grid_transpose_kernel(const V* __restrict__ src, V* __restrict__ dst,
+                                                                  uint32_t B, uint32_t L, uint32_t tile) {
+  extern __shared__ __align__(16) unsigned char tile_mem[];
+  V* sm = reinterpret_cast<V*>(tile_mem);
+  const uint32_t row = L * U, pitch = row | 1u;  // odd pitch: a column's vectors on distinct banks
+  const size_t b0 = (size_t)blockIdx.x * tile;
+  const uint32_t n = (uint32_t)(B - b0 < tile ? B - b0 : tile);
+  const uint32_t per_level = n * U, total = per_level * L;
+  if (TO_ROWS) {
+    for (uint32_t i = threadIdx.x; i < total; i += kThreads) {
+      const uint32_t l = i / per_level, k = i - l * per_level;
+      sm[(k / U) * pitch + l * U + k % U] = src[((size_t)l * B + b0) * U + k];
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < total; i += kThreads) {
+      const uint32_t b = i / row;
+      dst[b0 * row + i] = sm[b * pitch + (i - b * row)];
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < total; i += kThreads) {
+      const uint32_t b = i / row;
+      sm[b * pitch + (i - b * row)] = src[b0 * row + i];
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < total; i += kThreads) {
+      const uint32_t l = i / per_level, k = i - l * per_level;
+      dst[((size_t)l * B + b0) * U + k] = sm[(k / U) * pitch + l * U + k % U];
+    }
+  }
+}
 
 bool aligned(const void* p, size_t bytes) { return ((uintptr_t)p % bytes) == 0; }
 
@@ -417,6 +458,41 @@ int check_geo(const Geo& g, const void* inputs, const int32_t* offsets) {
 }
 
 }  // namespace
+
+// Shared memory of one transposition block: 64 points or as many as fit 40 KB.
+constexpr size_t kTransposeSmem = 40 * 1024;
+
+template <typename V, int U>
+static int transpose_typed(const void* src, void* dst, uint32_t B, uint32_t L, bool to_rows, cudaStream_t st) {
+  const size_t per_point = ((size_t)L * U | 1u) * sizeof(V);
+  const uint32_t tile = (uint32_t)std::min<size_t>(64, kTransposeSmem / per_point);
+  const unsigned grid = (unsigned)(((size_t)B + tile - 1) / tile);
+  auto* k = to_rows ? grid_transpose_kernel<V, U, true> : grid_transpose_kernel<V, U, false>;
+  k<<<grid, kThreads, tile * per_point, st>>>((const V*)src, (V*)dst, B, L, tile);
+  return launch_error("grid transpose");
+}
+
+extern "C" int n3ds_grid_transpose(const void* src, void* dst, uint32_t B, uint32_t L, uint32_t unit_bytes,
+                                   int32_t to_rows, n3ds_stream_t stream) {
+  if (L < 1 || (unit_bytes != 2 && unit_bytes != 4 && unit_bytes != 8 && unit_bytes != 16 && unit_bytes != 32 &&
+                unit_bytes != 64))
+    return n3ds::report_error(N3DS_ERR_INVALID, "grid transpose: L >= 1 and units of 2 to 64 bytes required");
+  if ((size_t)L * unit_bytes + 16 > kTransposeSmem)
+    return n3ds::report_error(N3DS_ERR_UNSUPPORTED, "grid transpose: a row exceeds the shared-memory tile");
+  if (B == 0) return N3DS_OK;
+  const uint32_t v = unit_bytes < 16 ? unit_bytes : 16;
+  if (!src || !dst || !aligned(src, v) || !aligned(dst, v))
+    return n3ds::report_error(N3DS_ERR_INVALID, "grid transpose: aligned src and dst required");
+  const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  switch (unit_bytes) {
+    case 2: return transpose_typed<uint16_t, 1>(src, dst, B, L, to_rows != 0, st);
+    case 4: return transpose_typed<uint32_t, 1>(src, dst, B, L, to_rows != 0, st);
+    case 8: return transpose_typed<uint2, 1>(src, dst, B, L, to_rows != 0, st);
+    case 16: return transpose_typed<uint4, 1>(src, dst, B, L, to_rows != 0, st);
+    case 32: return transpose_typed<uint4, 2>(src, dst, B, L, to_rows != 0, st);
+    default: return transpose_typed<uint4, 4>(src, dst, B, L, to_rows != 0, st);
+  }
+}
 
 extern "C" int n3ds_grid_encode_forward(const float* inputs, const void* embeddings, const int32_t* offsets,
                                         void* outputs, uint32_t B, uint32_t D, uint32_t C, uint32_t L, float S,

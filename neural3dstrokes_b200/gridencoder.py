@@ -141,6 +141,31 @@ def grad_total_variation(inputs, embeddings, grad, offsets, weight, B, D, C, L, 
             float(S), int(H), int(gridtype), int(bool(align_corners)), _dtype(embeddings), _lib.stream_ptr()))
 
 
+_TRANSPOSE_ROW_BYTES = 32 << 10  # rows up to this size go through the tiled transposition
+
+
+def _rows_of_levels(t, B, L, C):
+    """[L, B, C] -> [B, L * C] (contiguous)."""
+    unit = C * t.element_size()
+    if L == 1 or L * unit > _TRANSPOSE_ROW_BYTES or t.data_ptr() % min(unit, 16):
+        return t.permute(1, 0, 2).reshape(B, L * C)
+    out = torch.empty(B, L * C, device=t.device, dtype=t.dtype)
+    with torch.cuda.device(t.device):
+        _lib.check(_lib.load().n3ds_grid_transpose(_lib.ptr(t), _lib.ptr(out), B, L, unit, 1, _lib.stream_ptr()))
+    return out
+
+
+def _levels_of_rows(t, B, L, C):
+    """[B, L * C] -> [L, B, C] (contiguous)."""
+    unit = C * t.element_size()
+    if L == 1 or L * unit > _TRANSPOSE_ROW_BYTES or not t.is_contiguous() or t.data_ptr() % min(unit, 16):
+        return t.view(B, L, C).permute(1, 0, 2).contiguous()
+    out = torch.empty(L, B, C, device=t.device, dtype=t.dtype)
+    with torch.cuda.device(t.device):
+        _lib.check(_lib.load().n3ds_grid_transpose(_lib.ptr(t), _lib.ptr(out), B, L, unit, 0, _lib.stream_ptr()))
+    return out
+
+
 def _autocast_on():
     try:
         return torch.is_autocast_enabled("cuda")
@@ -168,7 +193,7 @@ class _grid_encode(torch.autograd.Function):
         dy_dx = torch.empty(B, L * D * C, device=inputs.device, dtype=embeddings.dtype) if calc_grad_inputs else None
         grid_encode_forward(inputs, embeddings, offsets, outputs, B, D, C, L, S, H, dy_dx, gridtype, align_corners,
                             interpolation)
-        outputs = outputs.permute(1, 0, 2).reshape(B, L * C)
+        outputs = _rows_of_levels(outputs, B, L, C)
         ctx.save_for_backward(inputs, embeddings, offsets, dy_dx)
         ctx.dims = [B, D, C, L, S, H, gridtype, interpolation]
         ctx.align_corners = align_corners
@@ -179,7 +204,7 @@ class _grid_encode(torch.autograd.Function):
     def backward(ctx, grad):
         inputs, embeddings, offsets, dy_dx = ctx.saved_tensors
         B, D, C, L, S, H, gridtype, interpolation = ctx.dims
-        grad = grad.view(B, L, C).permute(1, 0, 2).contiguous().to(embeddings.dtype)
+        grad = _levels_of_rows(grad, B, L, C).to(embeddings.dtype)
         grad_embeddings = torch.zeros_like(embeddings)
         grad_inputs = torch.zeros_like(inputs, dtype=embeddings.dtype) if dy_dx is not None else None
         grid_encode_backward(grad, inputs, embeddings, offsets, grad_embeddings, B, D, C, L, S, H, dy_dx,
