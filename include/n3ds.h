@@ -534,6 +534,13 @@ int n3ds_density_net_forward(const n3ds_density_net_t* net, const float* coords,
 int n3ds_density_net_backward(const n3ds_density_net_t* net, const float* coords, const float* features,
                               const float* grad_density, int64_t n_points, float* grad_table, float* grad_w1,
                               float* grad_b1, float* grad_w2, float* grad_b2, n3ds_stream_t stream);
+/* The same with a scratch of n_points * stride floats (16-byte aligned) for the feature
+ * gradients: the layers' adjoint and the table scatter then run as two kernels, each at its
+ * own occupancy. NULL: one kernel. */
+int n3ds_density_net_backward_scratch(const n3ds_density_net_t* net, const float* coords, const float* features,
+                                      const float* grad_density, int64_t n_points, float* grad_table, float* grad_w1,
+                                      float* grad_b1, float* grad_w2, float* grad_b2, float* scratch,
+                                      n3ds_stream_t stream);
 /* Hash-decay statistics of a float32 table (source/models.py:472-488):
  * out[l, c] = mean over level l's rows of table[row, c]^2, for every channel when
  * all_channels is nonzero (torch_scatter's segment_coo), else for channel 0 with

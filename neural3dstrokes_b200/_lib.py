@@ -127,6 +127,7 @@ _SIGS = {
     "n3ds_density_net_resident_ctas": (ctypes.c_int, [c_i32]),
     "n3ds_density_net_forward": (ctypes.c_int, [_DN, _P, c_i64, _P, _P, _P, _P]),
     "n3ds_density_net_backward": (ctypes.c_int, [_DN, _P, _P, _P, c_i64, _P, _P, _P, _P, _P, _P]),
+    "n3ds_density_net_backward_scratch": (ctypes.c_int, [_DN, _P, _P, _P, c_i64, _P, _P, _P, _P, _P, _P, _P]),
     "n3ds_grid_level_mean_sq": (ctypes.c_int, [_P, _P, c_u32, c_u32, c_i32, _P, _P]),
     "n3ds_grid_level_mean_sq_backward": (ctypes.c_int, [_P, _P, c_u32, c_u32, c_i32, _P, _P, _P]),
     "n3ds_stroke_forward_static": (ctypes.c_int, [_P, _P, _P, _P, c_i64, _P, _P, _P, _P, _P, c_i64, c_i64, c_i64,

@@ -61,20 +61,18 @@ constexpr int kStatusWait = 2;             // the field's ST_WAIT_TIMEOUT bit
 // Backward only, bf16:
 //   W1' = w2 (.) W1 in three terms: element (f, j) at (j / 8) * 256 + f * 16 + (j % 8) * 2
 //     (B of dfeat: N = f, K = hidden);
-//   ReLU mask rows: element (p, j) at (j / 8) * 2048 + p * 16 + (j % 8) * 2 (A of dfeat:
-//     M = points, K = hidden);
-//   ReLU mask transposed: element (j, p) at (j / 8) * 2304 + (j % 8) * 16 + (p / 8) * 144
-//     + (p % 8) * 2 (A of dW1: M = hidden, K = points);
-//   dr (.) feat in three terms, dr itself in column L*C: element (f, p) at (f / 8) * 2304
-//     + (f % 8) * 16 + (p / 8) * 144 + (p % 8) * 2 (B of dW1: N = f, K = points).
-// The transposed tiles are written a column per thread; their 144-byte K chunks (128 +
-// 16 of padding) put a warp's 32 columns on distinct banks.
+//   ReLU mask rows: element (p, j) at (j / 8) * 2048 + p * 16 + (j % 8) * 2: A of dfeat
+//     (M = points, K = hidden, K-major) and, read MN-major, A of dW1 (M = hidden, K = points);
+//   dr (.) feat in three terms, dr itself in column L*C: element (p, f) at (f / 8) * 2048
+//     + p * 16 + (f % 8) * 2 (B of dW1, MN-major: N = f, K = points).
+// Each thread writes its point's rows as 16-byte stores; the transposition that dW1 needs
+// is the operands' major-ness. (K-major transposed copies took 91 two-byte stores per point
+// and 19 KB more, which held the kernel at 3 CTAs per SM: layers' adjoint of PropMLP (2048)
+// on 2^20 points 149 us, 121 so.)
 constexpr uint32_t kW1pBytes = kMaxFeat * kHidden * 2;  // 2 KB per term
 constexpr uint32_t kMaskBytes = kTile * kHidden * 2;    // 16 KB
-constexpr uint32_t kPadChunk = 144, kPadGroup = 16 * kPadChunk;
-constexpr uint32_t kMaskTBytes = (kHidden / 8) * kPadGroup;   // 18 KB
-constexpr uint32_t kBpBytes = (kMaxFeat / 8) * kPadGroup;     // 4.5 KB per term
-struct Misc {
+constexpr uint32_t kBpBytes = kTile * kMaxFeat * 2;     // 4 KB per term
+struct alignas(16) Misc {
   float b1[kHidden];
   float w2[kHidden];
   Level lv[kMaxFeat];
@@ -85,7 +83,7 @@ struct Misc {
 // Offsets for kc 4-value feature chunks (2 when L * C <= 8, else 4): the feature and
 // W1 tiles hold only the chunks the first layer reads.
 struct Smem {
-  uint32_t feat_hi, feat_lo, w1_hi, w1_lo, w1p, mask, maskt, bp, misc_fwd, misc_bwd, fwd_bytes, bwd_bytes;
+  uint32_t feat_hi, feat_lo, w1_hi, w1_lo, w1p, mask, bp, misc_fwd, misc_bwd, fwd_bytes, bwd_bytes;
 };
 __host__ __device__ constexpr Smem smem_layout(int kc) {
   Smem m{};
@@ -96,8 +94,7 @@ __host__ __device__ constexpr Smem smem_layout(int kc) {
   m.w1p = m.w1_lo + kc * 1024;  // the forward's Misc, then the backward's tiles
   m.misc_fwd = m.w1p;
   m.mask = m.w1p + 3 * kW1pBytes;
-  m.maskt = m.mask + kMaskBytes;
-  m.bp = m.maskt + kMaskTBytes;
+  m.bp = m.mask + kMaskBytes;
   m.misc_bwd = m.bp + 3 * kBpBytes;
   m.fwd_bytes = m.misc_fwd + (uint32_t)sizeof(Misc);
   m.bwd_bytes = m.misc_bwd + (uint32_t)sizeof(Misc);
@@ -113,19 +110,20 @@ constexpr uint32_t kColsFwd = 64, kColsBwd = 128;
 
 constexpr uint32_t IDESC_L1 = idesc_tf32(kTile, kHidden, false, false);  // feat x W1, tf32
 constexpr uint32_t IDESC_DF = idesc_bf16(kTile, 16);                     // mask x W1', bf16
-constexpr uint32_t IDESC_DW = idesc_bf16(kHidden, 16);                   // mask^T x (dr feat), bf16
+constexpr uint32_t IDESC_DW = idesc_bf16(kHidden, 16) | IDESC_A_MN | IDESC_B_MN;  // mask^T x (dr feat), bf16
 
 struct NetLaunch {
   const float* coords;
   const float* table;
   const int32_t* offsets;
   const float *w1, *b1, *w2, *b2;
-  const float* features_in;  // backward: the forward's record
+  const float* features_in;  // the feature record (backward; the split forward's layers)
   const float* grad_density;
   float* density;
   float* features_out;       // forward: the record, or null
   float* coords_warped;
   float *g_table, *g_w1, *g_b1, *g_w2, *g_b2;
+  float* dfeat;              // split backward: feature gradients [n, stride]
   int32_t* status;
   long long n;
   uint32_t L, F, stride;     // levels, features (L * C), record floats per point
@@ -170,8 +168,33 @@ __device__ __forceinline__ void warp_point(const NetLaunch& P, float x0, float x
   for (int d = 0; d < 3; d++) u[d] = (w[d] + P.grid_bound) * P.inv_two_bound;
 }
 
-// L * C features of point u (grid_fwd_kernel's arithmetic, n3ds_grid.cu), zero when
-// u leaves [0, 1]^3 as in the reference.
+// The C features of point u (inside [0, 1]^3) at one level (grid_fwd_kernel's arithmetic,
+// n3ds_grid.cu).
+template <int C>
+__device__ __forceinline__ void encode_level(const NetLaunch& P, const Level& lv, const float (&u)[3], float (&res)[C]) {
+  const float* tab = P.table + (size_t)lv.base * C;
+  uint32_t cell[3];
+  float frac[3], deriv[3];
+  locate<3>(u, lv, P.align, false, cell, frac, deriv);
+  const bool pair_level = P.vec_pair && !(lv.base & 1u) && lv.hsize >= kPairMinRows;
+#pragma unroll
+  for (int c = 0; c < C; c++) res[c] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    uint32_t c0[3], c1[3];
+    const float w0 = corner_of<3>(2 * j, cell, frac, c0);
+    const float w1 = corner_of<3>(2 * j + 1, cell, frac, c1);
+    float v0[C], v1[C];
+    const uint32_t r0 = cell_row<3>(c0, lv, P.hash, P.align), r1 = cell_row<3>(c1, lv, P.hash, P.align);
+    load_rows2<float, C>(tab, r0, r1, P.vec_table, pair_level && (r0 | 1u) < lv.hsize, v0, v1);
+#pragma unroll
+    for (int c = 0; c < C; c++) res[c] += w0 * v0[c];
+#pragma unroll
+    for (int c = 0; c < C; c++) res[c] += w1 * v1[c];
+  }
+}
+
+// L * C features of point u, zero when u leaves [0, 1]^3 as in the reference.
 template <int C, int LMAX, bool EXACT>
 __device__ __forceinline__ void encode_point(const NetLaunch& P, const Level* lvs, const float (&u)[3],
                                              float (&f)[kMaxFeat]) {
@@ -181,28 +204,8 @@ __device__ __forceinline__ void encode_point(const NetLaunch& P, const Level* lv
 #pragma unroll
   for (int l = 0; l < LMAX; l++) {
     if (EXACT || l < (int)P.L) {  // EXACT: LMAX is the level count, no guard
-      const Level lv = lvs[l];
-      const float* tab = P.table + (size_t)lv.base * C;
-      uint32_t cell[3];
-      float frac[3], deriv[3];
-      locate<3>(u, lv, P.align, false, cell, frac, deriv);
-      const bool pair_level = P.vec_pair && !(lv.base & 1u) && lv.hsize >= kPairMinRows;
       float res[C];
-#pragma unroll
-      for (int c = 0; c < C; c++) res[c] = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        uint32_t c0[3], c1[3];
-        const float w0 = corner_of<3>(2 * j, cell, frac, c0);
-        const float w1 = corner_of<3>(2 * j + 1, cell, frac, c1);
-        float v0[C], v1[C];
-        const uint32_t r0 = cell_row<3>(c0, lv, P.hash, P.align), r1 = cell_row<3>(c1, lv, P.hash, P.align);
-        load_rows2<float, C>(tab, r0, r1, P.vec_table, pair_level && (r0 | 1u) < lv.hsize, v0, v1);
-#pragma unroll
-        for (int c = 0; c < C; c++) res[c] += w0 * v0[c];
-#pragma unroll
-        for (int c = 0; c < C; c++) res[c] += w1 * v1[c];
-      }
+      encode_level<C>(P, lvs[l], u, res);
 #pragma unroll
       for (int c = 0; c < C; c++) f[l * C + c] = res[c];
     }
@@ -337,10 +340,52 @@ __device__ __forceinline__ void teardown(const NetLaunch& P, Misc* M, uint32_t p
   if (threadIdx.x < 32) tmem_dealloc(M->tmem, cols);
 }
 
+// ------------------------------------------------------------ encoding and scatter alone
+
+// The grid half of the split network: one thread per point and 16-byte chunk of its
+// feature record (4 / C levels), 128 points x CH chunks per block. The gathers (and the
+// backward's atomics) are bound by their latency: beside the tensor-core layers they run
+// at 16 (12) warps per SM, held by registers and tensor memory; alone, at 64 registers,
+// at 32, with the record as the only extra traffic (32 bytes written and read per point).
+// PropMLP (2048) on 2^20 points: encode and layers in one kernel 306 us, split 148 + 37;
+// backward 450 us, split 121 + 263.
+template <int C, int CH>
+__global__ void __launch_bounds__(kTile * CH, CH == 1 ? 8 : CH == 2 ? 4 : CH == 3 ? 2 : 2) density_encode_kernel(const NetLaunch P) {
+  constexpr int NL = 4 / C;
+  __shared__ Level lvs[kMaxFeat];
+  if (threadIdx.x < P.L) lvs[threadIdx.x] = level_of(P.offsets, threadIdx.x, P.S, P.H);
+  __syncthreads();
+  const int chunk = threadIdx.x / kTile;
+  const long long b = (long long)blockIdx.x * kTile + threadIdx.x % kTile;
+  if (b >= P.n) return;
+  float w[3], u[3];
+  warp_point(P, P.coords[3 * b], P.coords[3 * b + 1], P.coords[3 * b + 2], w, u);
+  if (chunk == 0 && P.coords_warped) {
+    P.coords_warped[3 * b] = w[0];
+    P.coords_warped[3 * b + 1] = w[1];
+    P.coords_warped[3 * b + 2] = w[2];
+  }
+  float f[4] = {0.f, 0.f, 0.f, 0.f};
+  if (point_in_range(u, 3)) {
+#pragma unroll
+    for (int q = 0; q < NL; q++) {
+      const int l = chunk * NL + q;
+      if (l < (int)P.L) {  // warp-uniform
+        float res[C];
+        encode_level<C>(P, lvs[l], u, res);
+#pragma unroll
+        for (int c = 0; c < C; c++) f[q * C + c] = res[c];
+      }
+    }
+  }
+  *reinterpret_cast<float4*>(P.features_out + b * P.stride + 4 * chunk) = make_float4(f[0], f[1], f[2], f[3]);
+}
+
 // ------------------------------------------------------------ forward
 
-template <int C, int LMAX, bool EXACT>
-__global__ void __launch_bounds__(kTile, 4) density_fwd_kernel(NetLaunch P) {
+// ENC: encode the points here; else read the feature record density_encode_kernel wrote.
+template <int C, int LMAX, bool EXACT, bool ENC>
+__global__ void __launch_bounds__(kTile, ENC ? 4 : 8) density_fwd_kernel(NetLaunch P) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const Smem SL = smem_layout(P.F > 8 ? 4 : 2);
   Misc* M = reinterpret_cast<Misc*>(smem + SL.misc_fwd);
@@ -356,7 +401,20 @@ __global__ void __launch_bounds__(kTile, 4) density_fwd_kernel(NetLaunch P) {
     const long long b = tile * kTile + tid;
     const bool valid = b < P.n;
     float f[kMaxFeat];
-    {
+    if constexpr (!ENC) {
+#pragma unroll
+      for (int i = 0; i < kMaxFeat; i++) f[i] = 0.f;
+      if (valid) {
+        const float4* rec = reinterpret_cast<const float4*>(P.features_in + b * P.stride);
+#pragma unroll
+        for (int c = 0; c < kMaxFeat / 4; c++) {
+          if (c < (int)(P.stride / 4)) {
+            const float4 r = rec[c];
+            f[4 * c] = r.x; f[4 * c + 1] = r.y; f[4 * c + 2] = r.z; f[4 * c + 3] = r.w;
+          }
+        }
+      }
+    } else {
       float x[3] = {0.f, 0.f, 0.f}, w[3], u[3];
       if (valid) {
         x[0] = P.coords[3 * b];
@@ -419,12 +477,24 @@ __global__ void __launch_bounds__(kTile, 4) density_fwd_kernel(NetLaunch P) {
 
 // ------------------------------------------------------------ backward
 
+// Two rows of a one-channel level: one 8-byte atomic when they are an aligned pair (the
+// x-neighbours of a cell with even x), half the cells. At the scatter kernel's occupancy
+// the fewer atomics pay for the test (297 -> 262 us); beside the layers they do not.
+__device__ __forceinline__ void scatter_pair(float* tab, uint32_t r0, uint32_t r1, float v0, float v1, bool pair) {
+  if (pair && (r0 ^ r1) == 1u) {
+    atomicAdd(reinterpret_cast<float2*>(tab + (r0 & ~1u)), (r0 & 1u) ? make_float2(v1, v0) : make_float2(v0, v1));
+  } else {
+    atomicAdd(tab + r0, v0);
+    atomicAdd(tab + r1, v1);
+  }
+}
 // grad_table[corner rows of point u at level lv] += w * g, with runs of lanes in one
 // cell summed first (grid_bwd_kernel's scheme, n3ds_grid.cu). Every lane calls it.
-template <int C>
+template <int C, bool PAIR = false>
 __device__ __forceinline__ void scatter_level(const NetLaunch& P, const Level& lv, const float (&u)[3], bool valid,
                                               const float (&g)[C], int lane) {
   constexpr unsigned kFull = 0xffffffffu;
+  const bool pair = PAIR && P.vec_pair && !(lv.base & 1u) && !(lv.hsize & 1u);
   float* tab = P.g_table + (size_t)lv.base * C;
   uint32_t cell[3];
   float frac[3], deriv[3];
@@ -439,6 +509,16 @@ __device__ __forceinline__ void scatter_level(const NetLaunch& P, const Level& l
   const unsigned heads = __ballot_sync(kFull, head);
   if (heads == kFull) {
     if (!valid) return;
+    if constexpr (PAIR && C == 1) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        uint32_t c0[3], c1[3];
+        const float w0 = corner_of<3>(2 * j, cell, frac, c0), w1 = corner_of<3>(2 * j + 1, cell, frac, c1);
+        const uint32_t r0 = cell_row<3>(c0, lv, P.hash, P.align), r1 = cell_row<3>(c1, lv, P.hash, P.align);
+        scatter_pair(tab, r0, r1, w0 * g[0], w1 * g[0], pair);
+      }
+      return;
+    }
 #pragma unroll
     for (int corner = 0; corner < 8; corner++) {
       uint32_t cc[3];
@@ -487,7 +567,7 @@ struct BwdIn {
   float g;
   bool valid;
 };
-template <int FP>
+template <int FP, bool SCATTER>
 __device__ __forceinline__ void load_bwd_in(const NetLaunch& P, long long b, BwdIn<FP>& in) {
   in.valid = b < P.n;
   in.g = 0.f;
@@ -496,8 +576,10 @@ __device__ __forceinline__ void load_bwd_in(const NetLaunch& P, long long b, Bwd
 #pragma unroll
   for (int i = 0; i < FP; i++) in.f[i] = 0.f;
   if (!in.valid) return;
+  if (SCATTER) {
 #pragma unroll
-  for (int i = 0; i < 3; i++) in.x[i] = P.coords[3 * b + i];
+    for (int i = 0; i < 3; i++) in.x[i] = P.coords[3 * b + i];
+  }
   const float4* rec = reinterpret_cast<const float4*>(P.features_in + b * P.stride);
 #pragma unroll
   for (int c = 0; c < FP / 4; c++) {
@@ -509,15 +591,16 @@ __device__ __forceinline__ void load_bwd_in(const NetLaunch& P, long long b, Bwd
   in.g = P.grad_density[b];
 }
 
-template <int C, int LMAX, bool EXACT>
-__global__ void __launch_bounds__(kTile, 3) density_bwd_kernel(NetLaunch P) {
+// CTAs per SM: 4 (the tensor-memory limit) with 8 feature columns; 16 hold more registers.
+constexpr int FP_CTAS(int features) { return features <= 8 ? 4 : 3; }
+// SCATTER: scatter the feature gradients into the table here; else write them to P.dfeat
+// for density_scatter_kernel.
+template <int C, int LMAX, bool EXACT, bool SCATTER>
+__global__ void __launch_bounds__(kTile, SCATTER ? 3 : FP_CTAS(C * LMAX)) density_bwd_kernel(NetLaunch P) {
   constexpr int FP = C * LMAX <= 8 ? 8 : 16;
   extern __shared__ __align__(1024) uint8_t smem[];
   const Smem SL = smem_layout(P.F > 8 ? 4 : 2);
   Misc* M = reinterpret_cast<Misc*>(smem + SL.misc_bwd);
-  // the d raw (.) feat tile's columns beyond L * C (d raw itself) stay zero: cleared
-  // once here, the tiles write columns 0 .. L * C only
-  for (uint32_t i = threadIdx.x; i < 3 * kBpBytes / 4; i += kTile) reinterpret_cast<float*>(smem + SL.bp)[i] = 0.f;
   setup_cta(P, smem, SL, M, kColsBwd, true);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t tmem = M->tmem;
@@ -531,11 +614,9 @@ __global__ void __launch_bounds__(kTile, 3) density_bwd_kernel(NetLaunch P) {
   const uint32_t fh = smem_u32(smem + SL.feat_hi), fl = smem_u32(smem + SL.feat_lo);
   const uint32_t wh = smem_u32(smem + SL.w1_hi), wl = smem_u32(smem + SL.w1_lo);
   const uint32_t w1p = smem_u32(smem + SL.w1p), mask = smem_u32(smem + SL.mask);
-  const uint32_t maskt = smem_u32(smem + SL.maskt), bp = smem_u32(smem + SL.bp);
-  // this thread's column offset in the transposed tiles
-  const uint32_t col_off = (uint32_t)(tid / 8) * kPadChunk + (uint32_t)(tid % 8) * 2;
+  const uint32_t bp = smem_u32(smem + SL.bp);
   BwdIn<FP> in;
-  load_bwd_in<FP>(P, (long long)blockIdx.x * kTile + tid, in);
+  load_bwd_in<FP, SCATTER>(P, (long long)blockIdx.x * kTile + tid, in);
   for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     const bool valid = in.valid;
     const float g = in.g;
@@ -543,7 +624,7 @@ __global__ void __launch_bounds__(kTile, 3) density_bwd_kernel(NetLaunch P) {
     float f[FP];
 #pragma unroll
     for (int i = 0; i < FP; i++) f[i] = i < (int)P.F ? in.f[i] : 0.f;
-    if (valid) {
+    if (SCATTER && valid) {
       float w[3];
       warp_point(P, in.x[0], in.x[1], in.x[2], w, u);
     }
@@ -566,23 +647,8 @@ __global__ void __launch_bounds__(kTile, 3) density_bwd_kernel(NetLaunch P) {
       timed_out = true;
       break;
     }
-    // raw, then d raw through softplus
+    // raw, then d raw through softplus; the ReLU mask rows on the way
     float raw = M->b2;
-#pragma unroll
-    for (int c = 0; c < kHidden / 16; c++) {
-      float v[16];
-      tmem_ld16(lane_addr + COL_D1 + c * 16, v);
-#pragma unroll
-      for (int k = 0; k < 16; k++) raw = fmaf(relu_t(v[k] + M->b1[c * 16 + k]), M->w2[c * 16 + k], raw);
-    }
-    const float dr = P.raw_output ? g : softplus_backward_t(g, raw + P.density_bias);
-    {
-      float s = dr;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      acc_b2 += s;
-    }
-    // the ReLU mask (rows and transposed) and dW2 (warp sums of dr relu(pre))
 #pragma unroll
     for (int c = 0; c < kHidden / 16; c++) {
       float v[16];
@@ -591,34 +657,55 @@ __global__ void __launch_bounds__(kTile, 3) density_bwd_kernel(NetLaunch P) {
 #pragma unroll
       for (int k = 0; k < 16; k++) {
         const float pre = v[k] + M->b1[c * 16 + k];
+        raw = fmaf(relu_t(pre), M->w2[c * 16 + k], raw);
         // torch.relu's backward passes the gradient unless the output is <= 0 (NaN passes)
         const uint32_t one = pre <= 0.f ? 0u : 0x3F80u;
         if (k % 2 == 0) words[k / 2] = one;
         else words[k / 2] |= one << 16;
-        const int j = c * 16 + k;
-        *reinterpret_cast<uint16_t*>(smem + SL.maskt + (j / 8) * kPadGroup + (j % 8) * 16 + col_off) =
-            (uint16_t)one;
-        v[k] = dr * relu_t(pre);
       }
       *reinterpret_cast<uint4*>(smem + SL.mask + (2 * c) * 2048 + tid * 16) =
           make_uint4(words[0], words[1], words[2], words[3]);
       *reinterpret_cast<uint4*>(smem + SL.mask + (2 * c + 1) * 2048 + tid * 16) =
           make_uint4(words[4], words[5], words[6], words[7]);
+    }
+    const float dr = P.raw_output ? g : softplus_backward_t(g, raw + P.density_bias);
+    {
+      float s = dr;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      acc_b2 += s;
+    }
+    // dW2: warp sums of dr relu(pre). (The dW1 product holds it too, as W1 . dW1 sums, but
+    // its tensor-core accumulation rounds towards zero: 1.4e-5 of the norm, 9e-7 so.)
+#pragma unroll
+    for (int c = 0; c < kHidden / 16; c++) {
+      float v[16];
+      tmem_ld16(lane_addr + COL_D1 + c * 16, v);
+#pragma unroll
+      for (int k = 0; k < 16; k++) v[k] = dr * relu_t(v[k] + M->b1[c * 16 + k]);
       acc_w2[c] += warp_slot_sum16(v, lane);
     }
-    // dr (.) feat and dr (column L * C), three bf16 terms, transposed
-    auto put_bp = [&](int i, float x) {
-      uint16_t t[3];
-      split3_bf16(x, t[0], t[1], t[2]);
-      const uint32_t o = (i / 8) * kPadGroup + (i % 8) * 16 + col_off;
+    // dr (.) feat and dr (column L * C), three bf16 terms; f is 0 beyond L * C
 #pragma unroll
-      for (int k = 0; k < 3; k++) *reinterpret_cast<uint16_t*>(smem + SL.bp + k * kBpBytes + o) = t[k];
-    };
+    for (int h = 0; h < kMaxFeat / 8; h++) {
+      uint32_t words[3][4];
 #pragma unroll
-    for (int i = 0; i < FP; i++) {
-      if (i < (int)P.F) put_bp(i, dr * f[i]);
+      for (int i = 0; i < 8; i++) {
+        const int col = 8 * h + i;
+        const float x = col == (int)P.F ? dr : (col < FP ? dr * f[col < FP ? col : 0] : 0.f);
+        uint16_t t[3];
+        split3_bf16(x, t[0], t[1], t[2]);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          if (i % 2 == 0) words[k][i / 2] = t[k];
+          else words[k][i / 2] |= (uint32_t)t[k] << 16;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        *reinterpret_cast<uint4*>(smem + SL.bp + k * kBpBytes + h * 2048 + tid * 16) =
+            make_uint4(words[k][0], words[k][1], words[k][2], words[k][3]);
     }
-    put_bp((int)P.F, dr);
     fence_proxy_async();
     tc_fence_before_sync();
     __syncthreads();
@@ -633,23 +720,34 @@ __global__ void __launch_bounds__(kTile, 3) density_bwd_kernel(NetLaunch P) {
       }
       // mask^T . (dr feat) (M 64 hidden, N 16, K 128 points), accumulated over tiles
       for (int ks = 0; ks < kTile / 16; ks++) {
-        const uint64_t a = smem_desc(maskt + ks * 2 * kPadChunk, kPadChunk, kPadGroup);
+        const uint64_t a = smem_desc(mask + ks * 256, 128, 2048);
 #pragma unroll
         for (int t = 0; t < 3; t++)
-          mma_bf16(tmem + COL_DW, a, smem_desc(bp + t * kBpBytes + ks * 2 * kPadChunk, kPadChunk, kPadGroup),
-                   IDESC_DW, any || ks > 0 || t > 0);
+          mma_bf16(tmem + COL_DW, a, smem_desc(bp + t * kBpBytes + ks * 256, 128, 2048), IDESC_DW,
+                   any || ks > 0 || t > 0);
       }
       mma_commit(&M->bar);
     }
     any = true;
     // the next tile's inputs, fetched while the tensor cores work and the scatter runs
-    load_bwd_in<FP>(P, (tile + gridDim.x) * kTile + tid, in);
+    load_bwd_in<FP, SCATTER>(P, (tile + gridDim.x) * kTile + tid, in);
     if (!wait_mma(P, M, phase)) {
       timed_out = true;
       break;
     }
     float df[16];
     tmem_ld16(lane_addr + COL_DF, df);
+    if constexpr (!SCATTER) {
+      if (valid) {
+        float4* out = reinterpret_cast<float4*>(P.dfeat + (tile * kTile + tid) * P.stride);
+#pragma unroll
+        for (int c = 0; c < FP / 4; c++) {
+          if (c < (int)(P.stride / 4))
+            out[c] = make_float4(dr * df[4 * c], dr * df[4 * c + 1], dr * df[4 * c + 2], dr * df[4 * c + 3]);
+        }
+      }
+      continue;
+    }
     const bool in_grid = valid && point_in_range(u, 3);
 #pragma unroll
     for (int l = 0; l < LMAX; l++) {
@@ -680,6 +778,37 @@ __global__ void __launch_bounds__(kTile, 3) density_bwd_kernel(NetLaunch P) {
     if (lane == 0) atomicAdd(P.g_b2, acc_b2);
   }
   teardown(P, M, phase, timed_out, kColsBwd);
+}
+
+// The table scatter of the split backward: the feature gradients of one point and chunk.
+template <int C, int CH>
+__global__ void __launch_bounds__(kTile * CH) density_scatter_kernel(const NetLaunch P) {
+  constexpr int NL = 4 / C;
+  __shared__ Level lvs[kMaxFeat];
+  if (threadIdx.x < P.L) lvs[threadIdx.x] = level_of(P.offsets, threadIdx.x, P.S, P.H);
+  __syncthreads();
+  const int chunk = threadIdx.x / kTile, lane = threadIdx.x & 31;
+  const long long b = (long long)blockIdx.x * kTile + threadIdx.x % kTile;
+  float u[3] = {0.f, 0.f, 0.f};
+  float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool in_grid = b < P.n;
+  if (in_grid) {
+    float w[3];
+    warp_point(P, P.coords[3 * b], P.coords[3 * b + 1], P.coords[3 * b + 2], w, u);
+    in_grid = point_in_range(u, 3);
+    if (in_grid) g = *reinterpret_cast<const float4*>(P.dfeat + b * P.stride + 4 * chunk);
+  }
+  const float gv[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+  for (int q = 0; q < NL; q++) {
+    const int l = chunk * NL + q;
+    if (l < (int)P.L) {  // warp-uniform
+      float gl[C];
+#pragma unroll
+      for (int c = 0; c < C; c++) gl[c] = gv[q * C + c];
+      scatter_level<C, true>(P, lvs[l], u, in_grid, gl, lane);
+    }
+  }
 }
 
 // ------------------------------------------------------------ hash-decay statistics
@@ -906,29 +1035,52 @@ int resident(K kernel, uint32_t smem_max, uint32_t smem, uint32_t cols, int* cac
 
 int g_resident[2];  // CTAs of the last forward and backward launch
 
-template <int C, int LMAX, bool EXACT>
+template <int C>
+int launch_encode(const NetLaunch& P, cudaStream_t st) {
+  const unsigned blocks = (unsigned)((P.n + kTile - 1) / kTile);
+  switch (P.stride / 4) {
+    case 1: density_encode_kernel<C, 1><<<blocks, kTile, 0, st>>>(P); break;
+    case 2: density_encode_kernel<C, 2><<<blocks, 2 * kTile, 0, st>>>(P); break;
+    case 3: density_encode_kernel<C, 3><<<blocks, 3 * kTile, 0, st>>>(P); break;
+    default: density_encode_kernel<C, 4><<<blocks, 4 * kTile, 0, st>>>(P); break;
+  }
+  return launch_error("density net encoding");
+}
+template <int C>
+int launch_scatter(const NetLaunch& P, cudaStream_t st) {
+  const unsigned blocks = (unsigned)((P.n + kTile - 1) / kTile);
+  switch (P.stride / 4) {
+    case 1: density_scatter_kernel<C, 1><<<blocks, kTile, 0, st>>>(P); break;
+    case 2: density_scatter_kernel<C, 2><<<blocks, 2 * kTile, 0, st>>>(P); break;
+    case 3: density_scatter_kernel<C, 3><<<blocks, 3 * kTile, 0, st>>>(P); break;
+    default: density_scatter_kernel<C, 4><<<blocks, 4 * kTile, 0, st>>>(P); break;
+  }
+  return launch_error("density net scatter");
+}
+
+template <int C, int LMAX, bool EXACT, bool ENC>
 int fwd_c(const NetLaunch& P, cudaStream_t st) {
   static int cache[2][16] = {{0}};
   const int kc = P.F > 8 ? 4 : 2;
   const uint32_t smem = smem_layout(kc).fwd_bytes;
-  const int slots = resident(density_fwd_kernel<C, LMAX, EXACT>, smem_layout(4).fwd_bytes, smem, kColsFwd, cache[kc / 4]);
+  const int slots = resident(density_fwd_kernel<C, LMAX, EXACT, ENC>, smem_layout(4).fwd_bytes, smem, kColsFwd, cache[kc / 4]);
   g_resident[0] = slots;
   const long long tiles = (P.n + kTile - 1) / kTile;
   const int grid = (int)(tiles < slots ? tiles : slots);
-  density_fwd_kernel<C, LMAX, EXACT><<<grid, kTile, smem, st>>>(P);
+  density_fwd_kernel<C, LMAX, EXACT, ENC><<<grid, kTile, smem, st>>>(P);
   return launch_error("density net forward");
 }
 
-template <int C, int LMAX, bool EXACT>
+template <int C, int LMAX, bool EXACT, bool SCATTER>
 int bwd_c(const NetLaunch& P, cudaStream_t st) {
   static int cache[2][16] = {{0}};
   const int kc = P.F > 8 ? 4 : 2;
   const uint32_t smem = smem_layout(kc).bwd_bytes;
-  const int slots = resident(density_bwd_kernel<C, LMAX, EXACT>, smem_layout(4).bwd_bytes, smem, kColsBwd, cache[kc / 4]);
+  const int slots = resident(density_bwd_kernel<C, LMAX, EXACT, SCATTER>, smem_layout(4).bwd_bytes, smem, kColsBwd, cache[kc / 4]);
   g_resident[1] = slots;
   const long long tiles = (P.n + kTile - 1) / kTile;
   const int grid = (int)(tiles < slots ? tiles : slots);
-  density_bwd_kernel<C, LMAX, EXACT><<<grid, kTile, smem, st>>>(P);
+  density_bwd_kernel<C, LMAX, EXACT, SCATTER><<<grid, kTile, smem, st>>>(P);
   return launch_error("density net backward");
 }
 
@@ -936,9 +1088,26 @@ int bwd_c(const NetLaunch& P, cudaStream_t st) {
 // networks (PropMLP 6 and 8 levels x 1 channel, ErrorMLP 5 x 2; unguarded level loops,
 // so every level's gathers can be in flight together), else a bound (8 or 15 levels
 // for C = 1, 7 for C = 2, 3 for C = 4) with a guard per level.
+// The split forms need the feature record (forward) or a scratch for the feature gradients
+// (backward). Forward: from 2^15 points at one channel and 2^18 at more, where the extra
+// launch and the record's traffic are paid for (PropMLP (2048) 29 / 26 us at 2^16 points
+// in one kernel / split, 292 / 181 at 2^20; ErrorMLP, 2 channels, 25 / 25 and 166 / 155).
+// Backward: whenever the caller gives the scratch (worth it from 2^19 points at one channel,
+// 2^16 at more: PropMLP (2048) 141 / 142 us at 2^18, 448 / 397 at 2^20; ErrorMLP 66 / 64 at
+// 2^16, 384 / 330 at 2^20). The layers alone depend on the feature count, 8 or 16 columns.
 template <bool BWD, int C, int LMAX, bool EXACT>
 int launch_net(const NetLaunch& P, cudaStream_t st) {
-  return BWD ? bwd_c<C, LMAX, EXACT>(P, st) : fwd_c<C, LMAX, EXACT>(P, st);
+  if (BWD && P.dfeat) {
+    const int rc = P.F <= 8 ? bwd_c<1, 8, false, false>(P, st) : bwd_c<1, 15, false, false>(P, st);
+    return rc ? rc : launch_scatter<C>(P, st);
+  }
+  if (!BWD && P.features_out && P.n >= (C == 1 ? 1 << 15 : 1 << 18)) {
+    if (const int rc = launch_encode<C>(P, st)) return rc;
+    NetLaunch Q = P;
+    Q.features_in = P.features_out;
+    return fwd_c<1, 1, false, false>(Q, st);
+  }
+  return BWD ? bwd_c<C, LMAX, EXACT, true>(P, st) : fwd_c<C, LMAX, EXACT, true>(P, st);
 }
 template <bool BWD>
 int dispatch_net(const NetLaunch& P, uint32_t C, cudaStream_t st) {
@@ -993,14 +1162,25 @@ extern "C" int n3ds_density_net_backward(const n3ds_density_net_t* net, const fl
                                          const float* grad_density, int64_t n_points, float* grad_table,
                                          float* grad_w1, float* grad_b1, float* grad_w2, float* grad_b2,
                                          n3ds_stream_t stream) {
+  return n3ds_density_net_backward_scratch(net, coords, features, grad_density, n_points, grad_table, grad_w1, grad_b1,
+                                           grad_w2, grad_b2, nullptr, stream);
+}
+
+extern "C" int n3ds_density_net_backward_scratch(const n3ds_density_net_t* net, const float* coords,
+                                                 const float* features, const float* grad_density, int64_t n_points,
+                                                 float* grad_table, float* grad_w1, float* grad_b1, float* grad_w2,
+                                                 float* grad_b2, float* scratch, n3ds_stream_t stream) {
   if (int rc = check_net(net, n_points)) return rc;
   if (n_points == 0) return N3DS_OK;
   if (!coords || !features || !grad_density || !grad_table || !grad_w1 || !grad_b1 || !grad_w2 || !grad_b2)
     return n3ds::report_error(N3DS_ERR_INVALID, "density net backward: every input and gradient pointer is required");
   if (!aligned(features, 16))
     return n3ds::report_error(N3DS_ERR_INVALID, "density net: the feature record must be 16-byte aligned");
+  if (scratch && !aligned(scratch, 16))
+    return n3ds::report_error(N3DS_ERR_INVALID, "density net: the scratch must be 16-byte aligned");
   NetLaunch P = make_launch(net, coords, n_points);
   P.features_in = features;
+  P.dfeat = scratch;
   P.grad_density = grad_density;
   P.g_table = grad_table;
   P.g_w1 = grad_w1;
@@ -1009,6 +1189,7 @@ extern "C" int n3ds_density_net_backward(const n3ds_density_net_t* net, const fl
   P.g_b2 = grad_b2;
   const size_t vw = net->level_dim * 4 < 16 ? net->level_dim * 4 : 16;
   P.vec_table = vw > 4 && aligned(grad_table, vw);
+  P.vec_pair = aligned(grad_table, 8);
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   return dispatch_net<true>(P, net->level_dim, st);
 }

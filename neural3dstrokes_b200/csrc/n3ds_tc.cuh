@@ -8,8 +8,8 @@
 // matrices" of 8 rows x 16 bytes (4 tf32 or 8 bf16 values per row); element (mn, k) of
 // one K step (8 tf32 or 16 bf16 values, 32 bytes) at
 //   (mn % 8) * 16 + (mn / 8) * SBO + (k / V) * LBO + (k % V) * (16 / V) bytes,
-// V = 4 (tf32) or 8 (bf16). (MN-major tf32 operands exist only in a swizzled layout;
-// these kernels use K-major operands throughout.)
+// V = 4 (tf32) or 8 (bf16). bf16 operands may also be MN-major (IDESC_A_MN below; MN-major
+// tf32 operands exist only in a swizzled layout).
 #pragma once
 #include <cstdint>
 
@@ -117,6 +117,11 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
          | ((uint32_t)(N >> 3) << 17)  // N / 8
          | ((uint32_t)(M >> 4) << 24); // M / 16
 }
+
+// A or B of an instruction descriptor MN-major: core matrices of 8 MN values (16 bytes) x
+// 8 K rows, element (mn, k) of one bf16 K step at
+//   (mn % 8) * 2 + (mn / 8) * SBO + (k % 8) * 16 + (k / 8) * LBO bytes.
+constexpr uint32_t IDESC_A_MN = 1u << 15, IDESC_B_MN = 1u << 16;
 
 // D[tmem] (+)= A * B^T over one K = 16 step of bf16 operands; issued by one thread.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,

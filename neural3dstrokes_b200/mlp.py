@@ -35,6 +35,11 @@ from . import _lib
 from .gridencoder import GridEncoder
 
 WARP_SCALE, WARP_CONTRACT, WARP_NONE = 0, 1, 2
+# Points per call for which memory is taken so that the encoding and the table scatter run
+# as kernels of their own (where these are faster, n3ds_propnet.cu; at most 1 GB): a feature
+# record in a forward that no backward follows, a scratch for the feature gradients.
+_SPLIT_FORWARD = (1 << 15, 1 << 24)
+_SPLIT_BACKWARD = {1: (1 << 19, 1 << 24), 2: (1 << 16, 1 << 24), 4: (1 << 16, 1 << 24)}  # by channels
 HIDDEN = 64
 
 
@@ -94,7 +99,9 @@ class _DensityNetFn(torch.autograd.Function):
         dev = x.device
         density = torch.empty(n, device=dev, dtype=torch.float32)
         warped = torch.empty(n, 3, device=dev, dtype=torch.float32)
-        feats = torch.empty(n, stride, device=dev, dtype=torch.float32) if need else None
+        # the record also carries the features from the encoding to the layers' kernel
+        keep = need or _SPLIT_FORWARD[0] <= n <= _SPLIT_FORWARD[1]
+        feats = torch.empty(n, stride, device=dev, dtype=torch.float32) if keep else None
         net = _net_struct(enc, w1, b1, w2, b2, density_bias, warp, bbox_size, raw_output, **opts)
         with torch.cuda.device(dev):
             _lib.check(lib.n3ds_density_net_forward(ctypes.byref(net), _lib.ptr(x), n, _lib.ptr(density),
@@ -102,7 +109,7 @@ class _DensityNetFn(torch.autograd.Function):
         ctx.mark_non_differentiable(warped)
         ctx.spec = spec
         ctx.shape = coords.shape[:-1]
-        ctx.save_for_backward(x, feats, embeddings, w1, b1, w2, b2)
+        ctx.save_for_backward(x, feats if need else None, embeddings, w1, b1, w2, b2)
         return density.reshape(ctx.shape), warped.reshape(coords.shape)
 
     @staticmethod
@@ -113,10 +120,12 @@ class _DensityNetFn(torch.autograd.Function):
         grads = [torch.zeros_like(t) for t in (embeddings, w1, b1, w2, b2)]
         net = _net_struct(enc, w1, b1, w2, b2, density_bias, warp, bbox_size, raw_output, **opts)
         lib = _lib.load()
+        lo, hi = _SPLIT_BACKWARD[embeddings.shape[1]]
+        scratch = torch.empty_like(feats) if lo <= x.shape[0] <= hi else None
         with torch.cuda.device(x.device):
-            _lib.check(lib.n3ds_density_net_backward(ctypes.byref(net), _lib.ptr(x), _lib.ptr(feats), _lib.ptr(g),
-                                                     x.shape[0], *[_lib.ptr(t) for t in grads],
-                                                     _lib.stream_ptr()))
+            _lib.check(lib.n3ds_density_net_backward_scratch(
+                ctypes.byref(net), _lib.ptr(x), _lib.ptr(feats), _lib.ptr(g), x.shape[0],
+                *[_lib.ptr(t) for t in grads], _lib.ptr(scratch), _lib.stream_ptr()))
         return (None,) + tuple(grads) + (None,)
 
 

@@ -408,3 +408,49 @@ def test_nan_coordinates_propagate_as_in_the_reference(cuda):
         fin = ~torch.isnan(b)
         if bool(fin.any()):
             assert rel(a[fin], b[fin]) < GRAD_TOL
+
+
+@pytest.mark.parametrize("name,n", [("prop512_bbox", 32768), ("prop2048_contract", 32769 + 127),
+                                    ("error256_bbox", 262144 + 1), ("c4_contract", 262144 + 129)])
+def test_split_network_matches_one_kernel(cuda, name, n):
+    """Encoding and layers as two kernels (from the record sizes where the forward splits)
+    give the one-kernel density and record bit for bit, and the split backward (layers'
+    adjoint to a scratch, then the scatter) the one-kernel gradients to the rounding of
+    sums in another order; NaN and out-of-grid points included."""
+    import ctypes
+    from neural3dstrokes_b200 import _lib
+    lib, net = _lib.load(), make_net(name, cuda)
+    x = ray_points(cuda, (n + 63) // 64, 64, 1.6 if net.warp_fn is None else 3.0)[:n].contiguous()
+    x[5] = float("nan")
+    enc, lay = net.encoder, net.density_layer
+    params = [enc.embeddings, lay[0].weight, lay[0].bias, lay[2].weight, lay[2].bias]
+    s = mlp._net_struct(enc, *params[1:], net.density_bias, mlp._warp_mode(net.warp_fn, False), net.bbox_size, False)
+    stride = lib.n3ds_density_net_feature_stride(enc.num_levels, enc.level_dim)
+    feats, small = torch.empty(n, stride, device=cuda), torch.empty(n, stride, device=cuda)
+    dens, warped = [torch.full((n,), -1.0, device=cuda) for _ in range(3)], torch.empty(n, 3, device=cuda)
+
+    def forward(lo, hi, out, rec):
+        _lib.check(lib.n3ds_density_net_forward(ctypes.byref(s), _lib.ptr(x[lo:hi]), hi - lo, _lib.ptr(out[lo:hi]),
+                                                None if rec is None else _lib.ptr(rec[lo:hi]),
+                                                _lib.ptr(warped[lo:hi]), _lib.stream_ptr()))
+
+    forward(0, n, dens[0], feats)                       # split
+    forward(0, n, dens[1], None)                        # one kernel, no record
+    for lo in range(0, n, 8192):                        # one kernel with its record
+        forward(lo, min(n, lo + 8192), dens[2], small)
+    assert torch.equal(dens[0].isnan(), dens[1].isnan()) and torch.equal(feats.nan_to_num(), small.nan_to_num())
+    assert torch.equal(dens[0].nan_to_num(), dens[1].nan_to_num())
+    assert torch.equal(dens[0].nan_to_num(), dens[2].nan_to_num())
+    g = torch.randn(n, device=cuda, generator=torch.Generator(device=cuda).manual_seed(4))
+    g[5] = 0.0
+    x[5], feats[5] = 0.1, 0.0
+    out = []
+    for scratch in (None, torch.empty(n, stride, device=cuda)):
+        grads = [torch.zeros_like(p) for p in params]
+        _lib.check(lib.n3ds_density_net_backward_scratch(
+            ctypes.byref(s), _lib.ptr(x), _lib.ptr(feats), _lib.ptr(g), n, *[_lib.ptr(t) for t in grads],
+            _lib.ptr(scratch), _lib.stream_ptr()))
+        out.append(grads)
+    # float32 sums of n terms in two orders: sqrt(n) x 2^-24 relative to the largest sums
+    for a, b in zip(*out):
+        assert rel(a, b) < 4 * n ** 0.5 * 2.0 ** -24
