@@ -210,6 +210,9 @@ typedef struct n3ds_strokes {
    * that carries only their code. A stroke outside the hint is an unsupported kind
    * (status bit 1, NaN outputs). */
   uint32_t base_mask;
+  /* 1: sdf_delta may be NULL and every stroke has softness uniform_delta */
+  int32_t has_uniform_delta;
+  float uniform_delta;
 } n3ds_strokes_t;
 
 typedef struct n3ds_options {
@@ -274,6 +277,27 @@ int n3ds_field_backward(const n3ds_batch_t* batch, const n3ds_rays_t* rays,
                         float* grad_x, float* grad_shape, float* grad_color, float* grad_density,
                         float* grad_sdf_delta, void* workspace, size_t workspace_bytes,
                         n3ds_stream_t stream);
+
+/* What StrokeField.predict_density forms from the module's state before it evaluates
+ * (models.py:660-681), in one launch with the stroke count on the device:
+ * window [2] = (frozen, active): active = stroke_step, frozen = max(stroke_step -
+ * max_opt_strokes, 0), both capped by step_limit when has_limit; delta [n_strokes] = the
+ * softness, annealed from sdf_delta to sdf_delta_eval by active / max_num_strokes when
+ * training (float64, rounded to float32), else sdf_delta_eval; density [n_strokes] =
+ * density_params * density_scale; and, when x is given, x [n_coords] = coords *
+ * coord_scale. stroke_step: device int32 scalar. */
+typedef struct n3ds_module_state {
+  const int32_t* stroke_step;
+  int32_t max_opt_strokes, max_num_strokes;
+  int32_t has_limit, step_limit;
+  int32_t training;
+  double sdf_delta, sdf_delta_eval;
+  const float* density_params; /* [n_strokes] */
+  float density_scale;
+  float coord_scale;
+} n3ds_module_state_t;
+int n3ds_field_module_inputs(const n3ds_module_state_t* state, int64_t n_strokes, const float* coords, int64_t n_coords,
+                             int32_t* window, float* delta, float* density, float* x, n3ds_stream_t stream);
 
 /* Synchronously read (and clear) the device status word and the count of evaluated
  * (sample, stroke) pairs of the last forward (with options.count_pairs; else 0).

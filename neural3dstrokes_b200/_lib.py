@@ -3,6 +3,7 @@
 There is no CPU fallback: importing an operator without the built library raises.
 Build it with ``python -m neural3dstrokes_b200.build``.
 """
+import contextlib
 import ctypes
 import os
 import threading
@@ -39,7 +40,15 @@ class Strokes(ctypes.Structure):
     _fields_ = [("sdf_ids", ctypes.c_void_p), ("shape_params", ctypes.c_void_p), ("param_stride", c_i32),
                 ("color_params", ctypes.c_void_p), ("density", ctypes.c_void_p),
                 ("sdf_delta", ctypes.c_void_p), ("use_laplace_transform", c_i32),
-                ("inv_scale_radius", c_i32), ("stroke_window", ctypes.c_void_p), ("base_mask", ctypes.c_uint32)]
+                ("inv_scale_radius", c_i32), ("stroke_window", ctypes.c_void_p), ("base_mask", ctypes.c_uint32),
+                ("has_uniform_delta", c_i32), ("uniform_delta", ctypes.c_float)]
+
+
+class ModuleState(ctypes.Structure):
+    _fields_ = [("stroke_step", ctypes.c_void_p), ("max_opt_strokes", c_i32), ("max_num_strokes", c_i32),
+                ("has_limit", c_i32), ("step_limit", c_i32), ("training", c_i32), ("sdf_delta", ctypes.c_double),
+                ("sdf_delta_eval", ctypes.c_double), ("density_params", ctypes.c_void_p),
+                ("density_scale", ctypes.c_float), ("coord_scale", ctypes.c_float)]
 
 
 class Options(ctypes.Structure):
@@ -82,6 +91,7 @@ _SIGS = {
     "n3ds_field_backward": (ctypes.c_int, [ctypes.POINTER(Batch), ctypes.POINTER(Rays),
                                            ctypes.POINTER(Strokes), ctypes.POINTER(Options), _P, _P, _P,
                                            _P, _P, _P, _P, _P, _P, c_size_t, _P]),
+    "n3ds_field_module_inputs": (ctypes.c_int, [ctypes.POINTER(ModuleState), c_i64, _P, c_i64, _P, _P, _P, _P, _P]),
     "n3ds_field_read_status": (ctypes.c_int, [_P, ctypes.POINTER(c_i32), ctypes.POINTER(ctypes.c_uint64), _P]),
     "n3ds_adam_step": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, c_i64, ctypes.c_float, ctypes.c_float,
                                       ctypes.c_float, ctypes.c_float, _P, _P]),
@@ -170,18 +180,27 @@ def ptr(t):
     """Device pointer of a tensor, or None for None / empty tensors."""
     if t is None or t.numel() == 0:
         return None
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def device_guard(device):
+    """torch.cuda.device(device), free of charge where it is the current one."""
+    index = device.index
+    return _SAME_DEVICE if index is None or index == torch.cuda.current_device() else torch.cuda.device(index)
 
 
 def stream_ptr(device=None):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    return torch.cuda.current_stream(device).cuda_stream
 
 
 def workspace(nbytes, device):
     """A 256-byte aligned byte buffer from torch's caching allocator."""
     buf = torch.empty(max(int(nbytes), 1) + 256, dtype=torch.uint8, device=device)
     off = (-buf.data_ptr()) % 256
-    return buf[off:off + max(int(nbytes), 1)]
+    return buf[off:] if off else buf
 
 
 def default_options(**kw):

@@ -319,7 +319,7 @@ static int field_common(const n3ds_batch_t* batch, const n3ds_rays_t* rays, cons
   if (*R > 0 && !(rays->x ? rays->radius != nullptr : (rays->origins && rays->radii)))
     return fail(N3DS_ERR_INVALID, "rays: x and radius, or origins and radii (samples cast in-kernel), are required");
   if (!strokes || (*S > 0 && (!strokes->sdf_ids || !strokes->shape_params || !strokes->color_params ||
-                              !strokes->density || !strokes->sdf_delta)))
+                              !strokes->density || !(strokes->sdf_delta || strokes->has_uniform_delta))))
     return fail(N3DS_ERR_INVALID, "strokes: sdf_ids, shape_params, color_params, density, sdf_delta required");
   if (*S > 0 && (strokes->param_stride < 1 || strokes->param_stride > 64))
     return fail(N3DS_ERR_INVALID, "strokes: param_stride must be in [1, 64]");
@@ -361,6 +361,7 @@ static n3ds::PrepLaunch make_prep(const n3ds_strokes_t* s, long long S, const Re
   p.color_stride = 3;
   p.density = s->density;
   p.sdf_delta = s->sdf_delta;
+  p.uniform_delta = s->uniform_delta;
   p.use_laplace = s->use_laplace_transform;
   p.inv_scale_radius = s->inv_scale_radius;
   p.cull_m = rv.cull_m;
@@ -525,6 +526,7 @@ int n3ds_field_backward(const n3ds_batch_t* batch, const n3ds_rays_t* rays, cons
     F.shape_params = strokes->shape_params;
     F.param_stride = strokes->param_stride;
     F.sdf_delta = strokes->sdf_delta;
+    F.uniform_delta = strokes->uniform_delta;
     F.recs = reinterpret_cast<const float*>(ws + lay.recs);
     F.gslots = reinterpret_cast<const float*>(ws + lay.gslots);
     F.n_strokes = S;
@@ -539,6 +541,37 @@ int n3ds_field_backward(const n3ds_batch_t* batch, const n3ds_rays_t* rays, cons
     n3ds::launch_finalize(F, st);
     N3DS_CUDA_TRY(cudaGetLastError());
   }
+  return N3DS_OK;
+}
+
+int n3ds_field_module_inputs(const n3ds_module_state_t* state, int64_t n_strokes, const float* coords, int64_t n_coords,
+                             int32_t* window, float* delta, float* density, float* x, n3ds_stream_t stream) {
+  if (!state || !state->stroke_step || !window || n_strokes < 0 || n_coords < 0)
+    return fail(N3DS_ERR_INVALID, "module inputs: state, stroke_step, window and sizes >= 0 required");
+  if (n_strokes > 0 && (!state->density_params || !delta || !density))
+    return fail(N3DS_ERR_INVALID, "module inputs: density_params, delta and density required");
+  if (x && n_coords > 0 && !coords) return fail(N3DS_ERR_INVALID, "module inputs: coords required");
+  n3ds::ModuleInputs m{};
+  m.stroke_step = state->stroke_step;
+  m.max_opt = state->max_opt_strokes;
+  m.has_limit = state->has_limit;
+  m.limit = state->step_limit;
+  m.training = state->training;
+  m.inv_max = 1.0 / double(state->max_num_strokes);
+  m.delta0 = state->sdf_delta;
+  m.delta1 = state->sdf_delta_eval;
+  m.density_params = state->density_params;
+  m.density_scale = state->density_scale;
+  m.coords = coords;
+  m.coord_scale = state->coord_scale;
+  m.n_strokes = n_strokes;
+  m.n_coords = x ? n_coords : 0;
+  m.window = window;
+  m.delta = delta;
+  m.density = density;
+  m.x = x;
+  n3ds::launch_module_inputs(m, reinterpret_cast<cudaStream_t>(stream));
+  N3DS_CUDA_TRY(cudaGetLastError());
   return N3DS_OK;
 }
 

@@ -1263,6 +1263,43 @@ __device__ void catmull_param_grads(const float* prm, const float* gc, int compa
   out[13] = gc[13];
 }
 
+// ============================================================ module inputs
+
+// The stroke window, softness, scaled densities and warped coordinates of one
+// predict_density call. Launch bound: as torch operations these are 17 launches of a few
+// hundred elements, about 250 of the 490 us of a call's host time; here one.
+__global__ void module_inputs_kernel(const ModuleInputs M) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  int active = *M.stroke_step;
+  int frozen = max(active - M.max_opt, 0);
+  if (M.has_limit) {
+    active = min(active, M.limit);
+    frozen = min(frozen, M.limit);
+  }
+  if (i == 0) {
+    M.window[0] = frozen;
+    M.window[1] = active;
+  }
+  if (i < M.n_strokes) {
+    double d = M.delta1;
+    if (M.training) {  // each operation rounded, as the float64 tensor expression
+      const double frac = fmin(fmax(__dmul_rn((double)active, M.inv_max), 0.0), 1.0);
+      d = __dadd_rn(__dmul_rn(M.delta0, __dsub_rn(1.0, frac)), __dmul_rn(M.delta1, frac));
+    }
+    M.delta[i] = (float)d;
+    M.density[i] = M.density_params[i] * M.density_scale;
+  }
+  for (long long j = i; j < M.n_coords; j += (long long)gridDim.x * blockDim.x) M.x[j] = M.coords[j] * M.coord_scale;
+}
+
+void launch_module_inputs(const ModuleInputs& m, cudaStream_t st) {
+  const int bs = 256;
+  long long blocks = (m.n_strokes + bs - 1) / bs;
+  const long long cb = (m.n_coords + bs - 1) / bs;
+  blocks = blocks > cb ? blocks : (cb < 148 * 8 ? cb : (blocks > 148 * 8 ? blocks : 148 * 8));
+  module_inputs_kernel<<<(unsigned)(blocks > 0 ? blocks : 1), bs, 0, st>>>(m);
+}
+
 // ================================================================ launchers
 
 void launch_prep(const PrepLaunch& p, cudaStream_t st) {

@@ -144,6 +144,22 @@ struct FinalizeLaunch {
   int win_begin[MAX_SCENES_PER_LAUNCH + 1];
 };
 
+// n3ds_field_module_inputs.
+struct ModuleInputs {
+  const int* stroke_step;
+  int max_opt, has_limit, limit, training;
+  double inv_max, delta0, delta1;
+  const float* density_params;
+  float density_scale;
+  const float* coords;
+  float coord_scale;
+  long long n_strokes, n_coords;
+  int* window;
+  float* delta;
+  float* density;
+  float* x;
+};
+
 // Window state of stroke s: 0 active, 1 frozen (no gradient), 2 absent.
 __device__ __forceinline__ int window_state(const int* window, int n_win_scenes, const int* win_begin, long long s) {
   if (!window) return 0;
@@ -159,6 +175,7 @@ constexpr int ST_BAD_KIND = 1;
 constexpr int ST_WAIT_TIMEOUT = 2;
 
 void launch_prep(const PrepLaunch& p, cudaStream_t st);
+void launch_module_inputs(const ModuleInputs& m, cudaStream_t st);
 cudaError_t launch_seg_fwd(const SegLaunch& L, int grid, int warps, size_t smem, cudaStream_t st);
 cudaError_t launch_seg_bwd(const SegLaunch& L, int grid, int warps, size_t smem, cudaStream_t st);
 void launch_ray_fwd(const RayLaunch& L, cudaStream_t st);

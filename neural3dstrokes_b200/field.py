@@ -10,7 +10,6 @@ positions and every stroke parameter: shape (translation, rotation, scale, base
 parameters, Bezier control points and radii), colour, density and softness.
 """
 import ctypes
-import dataclasses
 from dataclasses import dataclass
 from typing import Optional, Sequence
 
@@ -53,11 +52,12 @@ class FieldOptions:
 
 
 class _Native:
-    """ctypes argument blocks for one call (kept alive for the call's duration)."""
+    """ctypes argument blocks for one call (kept alive for the call's duration).
+    ``delta`` [S], or None with ``uniform_delta``."""
 
     def __init__(self, scene_rays, scene_strokes, n_samples, x, radius, tdist, dirs, bg, bg_value, opaque,
                  sdf_ids, shape_params, color_params, density, delta, laplace, inv_scale, options, origins=None,
-                 radii=None, window=None):
+                 radii=None, window=None, uniform_delta=None):
         n = len(scene_rays)
         self.nr = (ctypes.c_int64 * n)(*[int(v) for v in scene_rays])
         self.ns = (ctypes.c_int32 * n)(*[int(v) for v in scene_strokes])
@@ -66,7 +66,8 @@ class _Native:
                               float(bg_value), int(bool(opaque)), _lib.ptr(origins), _lib.ptr(radii))
         self.strokes = _lib.Strokes(_lib.ptr(sdf_ids), _lib.ptr(shape_params), int(shape_params.shape[1]),
                                     _lib.ptr(color_params), _lib.ptr(density), _lib.ptr(delta), int(bool(laplace)),
-                                    int(bool(inv_scale)), _lib.ptr(window))
+                                    int(bool(inv_scale)), _lib.ptr(window), 0, int(uniform_delta is not None),
+                                    0.0 if uniform_delta is None else uniform_delta)
         self.opt = options.c()
 
     def ws_bytes(self):
@@ -79,20 +80,55 @@ def _f32(t, name):
     return t.contiguous()
 
 
+def _launch_forward(nat, R, dev, forward_only):
+    """rgb, acc, depth, and the workspace that the backward reads."""
+    if forward_only:  # no backward can follow
+        nat.opt.forward_only = 1
+    lib = _lib.load()
+    with _lib.device_guard(dev):
+        ws_bytes = nat.ws_bytes()
+        if ws_bytes == 0:
+            raise RuntimeError("invalid batch description")
+        ws = _lib.workspace(ws_bytes, dev)
+        rgb = torch.empty(R, 3, device=dev)
+        acc = torch.empty(R, device=dev)
+        depth = torch.empty(R, device=dev)
+        rc = lib.n3ds_field_forward(ctypes.byref(nat.batch), ctypes.byref(nat.rays), ctypes.byref(nat.strokes),
+                                    ctypes.byref(nat.opt), _lib.ptr(rgb), _lib.ptr(acc), _lib.ptr(depth),
+                                    _lib.ptr(ws), ws_bytes, _lib.stream_ptr(dev))
+    _lib.check(rc)
+    return rgb, acc, depth, ws, ws_bytes
+
+
+def _launch_backward(nat, dev, grads, gx, gshape, gcol, gden, gdel, ws, ws_bytes):
+    g = [t.contiguous().float() if t is not None else None for t in grads]
+    with _lib.device_guard(dev):
+        rc = _lib.load().n3ds_field_backward(
+            ctypes.byref(nat.batch), ctypes.byref(nat.rays), ctypes.byref(nat.strokes), ctypes.byref(nat.opt),
+            _lib.ptr(g[0]), _lib.ptr(g[1]), _lib.ptr(g[2]), _lib.ptr(gx), _lib.ptr(gshape), _lib.ptr(gcol),
+            _lib.ptr(gden), _lib.ptr(gdel), _lib.ptr(ws), ws_bytes, _lib.stream_ptr(dev))
+    _lib.check(rc)
+
+
 class _FieldFn(torch.autograd.Function):
+    """``delta``: a [S] tensor, or a float for every stroke."""
+
     @staticmethod
     def forward(ctx, x, radius, tdist, dirs, shape_params, color_params, density, delta, bg_t, sdf_ids,
                 scene_rays, scene_strokes, bg_value, opaque, laplace, inv_scale, options, origins=None, radii=None,
                 window=None):
+        ctx.set_materialize_grads(False)  # absent upstream gradients stay None: zero in the kernels
         R, N = tdist.shape[0], tdist.shape[1] - 1
         tdist, dirs = _f32(tdist, "tdist"), _f32(dirs, "dirs")
         if x is not None:
             x, radius = _f32(x, "x"), _f32(radius, "radius")
         else:  # samples cast in-kernel from the rays
             origins, radii = _f32(origins, "origins"), _f32(radii, "radii")
-        shape_params, color_params, density, delta = (
+        shape_params, color_params, density = (
             _f32(t, n) for t, n in ((shape_params, "shape_params"), (color_params, "color_params"),
-                                    (density, "density"), (delta, "sdf_delta")))
+                                    (density, "density")))
+        uniform = delta if isinstance(delta, float) else None
+        delta = None if uniform is not None else _f32(delta, "sdf_delta")
         if sdf_ids.dtype != torch.int32 or not sdf_ids.is_cuda:
             raise RuntimeError("sdf_ids must be a CUDA int32 tensor")
         sdf_ids = sdf_ids.contiguous()
@@ -101,56 +137,41 @@ class _FieldFn(torch.autograd.Function):
                 raise RuntimeError("stroke_window must be a CUDA int32 tensor of (frozen, active) per scene")
             window = window.contiguous()
         bg_c = _f32(bg_t, "bg") if bg_t is not None else None
-        # without any input that needs a gradient no backward can follow
-        fwd_opts = options if any(ctx.needs_input_grad) else dataclasses.replace(options, forward_only=True)
         nat = _Native(scene_rays, scene_strokes, N, x, radius, tdist, dirs, bg_c, bg_value, opaque, sdf_ids,
-                      shape_params, color_params, density, delta, laplace, inv_scale, fwd_opts, origins, radii,
-                      window)
-        lib = _lib.load()
-        dev = tdist.device
-        with torch.cuda.device(dev):
-            ws_bytes = nat.ws_bytes()
-            if ws_bytes == 0:
-                raise RuntimeError("invalid batch description")
-            ws = _lib.workspace(ws_bytes, dev)
-            rgb = torch.empty(R, 3, device=dev)
-            acc = torch.empty(R, device=dev)
-            depth = torch.empty(R, device=dev)
-            rc = lib.n3ds_field_forward(ctypes.byref(nat.batch), ctypes.byref(nat.rays), ctypes.byref(nat.strokes),
-                                        ctypes.byref(nat.opt), _lib.ptr(rgb), _lib.ptr(acc), _lib.ptr(depth),
-                                        _lib.ptr(ws), ws_bytes, _lib.stream_ptr())
-        _lib.check(rc)
+                      shape_params, color_params, density, delta, laplace, inv_scale, options, origins, radii,
+                      window, uniform)
+        rgb, acc, depth, ws, ws_bytes = _launch_forward(nat, R, tdist.device, not any(ctx.needs_input_grad))
         ctx.save_for_backward(x, radius, tdist, dirs, shape_params, color_params, density, delta, sdf_ids, origins,
                               radii, window)
         ctx.bg = bg_c
         ctx.ws, ctx.ws_bytes = ws, ws_bytes
-        ctx.meta = (scene_rays, scene_strokes, bg_value, opaque, laplace, inv_scale, options)
+        ctx.meta = (scene_rays, scene_strokes, bg_value, opaque, laplace, inv_scale, options, uniform)
         return rgb, acc, depth
 
     @staticmethod
     def backward(ctx, g_rgb, g_acc, g_depth):
         x, radius, tdist, dirs, shape_params, color_params, density, delta, sdf_ids, origins, radii, window = \
             ctx.saved_tensors
-        scene_rays, scene_strokes, bg_value, opaque, laplace, inv_scale, options = ctx.meta
+        scene_rays, scene_strokes, bg_value, opaque, laplace, inv_scale, options, uniform = ctx.meta
         N = tdist.shape[1] - 1
         nat = _Native(scene_rays, scene_strokes, N, x, radius, tdist, dirs, ctx.bg, bg_value, opaque, sdf_ids,
                       shape_params, color_params, density, delta, laplace, inv_scale, options, origins, radii,
-                      window)
+                      window, uniform)
         gx = torch.empty_like(x) if (x is not None and ctx.needs_input_grad[0]) else None
         gshape = torch.empty_like(shape_params)
         gcol = torch.empty_like(color_params)
         gden = torch.empty_like(density)
-        gdel = torch.empty_like(delta)
-        g = [t.contiguous().float() if t is not None else None for t in (g_rgb, g_acc, g_depth)]
-        lib = _lib.load()
-        with torch.cuda.device(tdist.device):
-            rc = lib.n3ds_field_backward(ctypes.byref(nat.batch), ctypes.byref(nat.rays), ctypes.byref(nat.strokes),
-                                         ctypes.byref(nat.opt), _lib.ptr(g[0]), _lib.ptr(g[1]), _lib.ptr(g[2]),
-                                         _lib.ptr(gx), _lib.ptr(gshape), _lib.ptr(gcol), _lib.ptr(gden),
-                                         _lib.ptr(gdel), _lib.ptr(ctx.ws), ctx.ws_bytes, _lib.stream_ptr())
-        _lib.check(rc)
+        gdel = torch.empty_like(delta) if delta is not None else None
+        _launch_backward(nat, tdist.device, (g_rgb, g_acc, g_depth), gx, gshape, gcol, gden, gdel, ctx.ws, ctx.ws_bytes)
         return (gx, None, None, None, gshape, gcol, gden, gdel, None, None, None, None, None, None, None, None,
                 None, None, None, None)
+
+
+def _softness(sdf_delta, S, dev):
+    if not torch.is_tensor(sdf_delta):
+        return float(sdf_delta)
+    delta = sdf_delta.to(dev, torch.float32)
+    return delta.expand(S) if delta.dim() == 0 else delta
 
 
 def render_strokes(x: torch.Tensor, radius: torch.Tensor, tdist: torch.Tensor, dirs: torch.Tensor,
@@ -176,12 +197,7 @@ def render_strokes(x: torch.Tensor, radius: torch.Tensor, tdist: torch.Tensor, d
     S = int(sdf_ids.numel())
     R = int(x.shape[0])
     dev = x.device
-    if torch.is_tensor(sdf_delta):
-        delta = sdf_delta.to(dev, torch.float32)
-        if delta.dim() == 0:
-            delta = delta.expand(S)
-    else:
-        delta = torch.full((S,), float(sdf_delta), device=dev)
+    delta = _softness(sdf_delta, S, dev)
     if scene_sizes is None:
         scene_sizes = [(R, S)]
     scene_rays = [int(a) for a, _ in scene_sizes]
@@ -216,12 +232,7 @@ def render_rays(origins: torch.Tensor, directions: torch.Tensor, radii: torch.Te
     dev = tdist.device
     if origins.shape != (R, 3) or directions.shape != (R, 3) or radii.numel() != R or tdist.dim() != 2:
         raise ValueError("expected origins / directions [R,3], radii [R], tdist [R,N+1]")
-    if torch.is_tensor(sdf_delta):
-        delta = sdf_delta.to(dev, torch.float32)
-        if delta.dim() == 0:
-            delta = delta.expand(S)
-    else:
-        delta = torch.full((S,), float(sdf_delta), device=dev)
+    delta = _softness(sdf_delta, S, dev)
     if scene_sizes is None:
         scene_sizes = [(R, S)]
     scene_rays = [int(a) for a, _ in scene_sizes]

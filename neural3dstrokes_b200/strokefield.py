@@ -26,7 +26,9 @@ What predict_density does, and how it is done here:
   with no gradient of their own and none into the coordinates;
 - ``density_scale`` (models.py:673) and the training-time ``sdf_delta`` annealing
   towards ``sdf_delta_eval`` (models.py:675-680), computed on the device in float64
-  and rounded to float32 as the reference's Python arithmetic is;
+  and rounded to float32 as the reference's Python arithmetic is; these, the window and
+  the bbox warp are one launch (n3ds_field_module_inputs) when the module's count is an
+  int32 device scalar and its settings host numbers;
 - 'over' composition (models.py:709), then compute_alpha_weights and
   volumetric_rendering with the background colour (models.py:206-235).
 
@@ -34,12 +36,15 @@ Returns rgb [R,3], acc [R] (opacity) and depth [R]. Constant-rgb colour, 'over'
 composition and no stroke texture (the reference configs' setting) run fused; other
 settings raise NotImplementedError (the drop-in ``_strokelib`` operators cover them).
 """
+import ctypes
 from typing import Optional
 
+import numpy as np
 import torch
 
+from . import _lib
 from . import strokes as _strokes
-from .field import FieldOptions, render_strokes
+from .field import FieldOptions, _f32, _launch_backward, _launch_forward, _Native, render_strokes
 
 
 def _contract(x):
@@ -86,6 +91,70 @@ def annealed_delta(field, window):
     return d.to(torch.float32)
 
 
+def _plain_state(field, coords, dev):
+    """The module's state is what the one-launch form reads: an int32 count and float32
+    densities on the coordinates' device, host numbers for the settings."""
+    step, den = field.stroke_step, field.density_params
+    return (torch.is_tensor(step) and step.is_cuda and step.device == dev and step.dtype == torch.int32 and
+            step.numel() == 1 and den.is_cuda and den.device == dev and den.dtype == torch.float32 and
+            coords.dtype == torch.float32 and
+            all(isinstance(v, (int, float)) for v in (field.density_scale, field.sdf_delta, field.sdf_delta_eval)))
+
+
+def _state_args(field):
+    limit = getattr(field, "stroke_step_limit", None)
+    return (int(field.max_opt_strokes), int(field.max_num_strokes), int(limit is not None),
+            0 if limit is None else int(limit), int(bool(field.training)), float(field.sdf_delta),
+            float(field.sdf_delta_eval), float(field.density_scale))
+
+
+class _ModuleFieldFn(torch.autograd.Function):
+    """The field on a module's raw state: the stroke window, annealed softness, scaled
+    densities and (``scale``) warped coordinates in one launch, then the fused render."""
+
+    @staticmethod
+    def forward(ctx, x, radius, tdist, dirs, shape_params, color_params, density_params, bg_t, sdf_ids, stroke_step,
+                state, scale, bg_value, opaque, laplace, inv_scale, options):
+        ctx.set_materialize_grads(False)  # absent upstream gradients stay None: zero in the kernels
+        dev = x.device
+        x, radius, tdist, dirs, shape_params, color_params, density_params = (
+            _f32(t, n) for t, n in ((x, "x"), (radius, "radius"), (tdist, "tdist"), (dirs, "dirs"),
+                                    (shape_params, "shape_params"), (color_params, "color_params"),
+                                    (density_params, "density")))
+        bg_c = _f32(bg_t, "bg") if bg_t is not None else None
+        R, N = tdist.shape[0], tdist.shape[1] - 1
+        S = density_params.shape[0]
+        window = torch.empty(1, 2, dtype=torch.int32, device=dev)
+        delta, density = torch.empty_like(density_params), torch.empty_like(density_params)
+        warped = x if scale is None else torch.empty_like(x)
+        max_opt, max_num, has_limit, limit, training, d0, d1, density_scale = state
+        m = _lib.ModuleState(_lib.ptr(stroke_step), max_opt, max_num, has_limit, limit, training, d0, d1,
+                             _lib.ptr(density_params), density_scale, 1.0 if scale is None else scale)
+        with _lib.device_guard(dev):
+            _lib.check(_lib.load().n3ds_field_module_inputs(
+                ctypes.byref(m), S, _lib.ptr(x), x.numel(), _lib.ptr(window), _lib.ptr(delta), _lib.ptr(density),
+                None if scale is None else _lib.ptr(warped), _lib.stream_ptr(dev)))
+        nat = _Native([R], [S], N, warped, radius, tdist, dirs, bg_c, bg_value, opaque, sdf_ids, shape_params,
+                      color_params, density, delta, laplace, inv_scale, options, window=window)
+        rgb, acc, depth, ws, ws_bytes = _launch_forward(nat, R, dev, not any(ctx.needs_input_grad))
+        ctx.save_for_backward(warped, radius, tdist, dirs, shape_params, color_params, density, delta, sdf_ids, window)
+        ctx.bg, ctx.ws, ctx.ws_bytes = bg_c, ws, ws_bytes
+        ctx.meta = (bg_value, opaque, laplace, inv_scale, options, density_scale)
+        return rgb, acc, depth
+
+    @staticmethod
+    def backward(ctx, g_rgb, g_acc, g_depth):
+        x, radius, tdist, dirs, shape_params, color_params, density, delta, sdf_ids, window = ctx.saved_tensors
+        bg_value, opaque, laplace, inv_scale, options, density_scale = ctx.meta
+        nat = _Native([tdist.shape[0]], [density.shape[0]], tdist.shape[1] - 1, x, radius, tdist, dirs, ctx.bg,
+                      bg_value, opaque, sdf_ids, shape_params, color_params, density, delta, laplace, inv_scale,
+                      options, window=window)
+        gx = torch.empty_like(x) if ctx.needs_input_grad[0] else None
+        gshape, gcol, gden = (torch.empty_like(t) for t in (shape_params, color_params, density))
+        _launch_backward(nat, tdist.device, (g_rgb, g_acc, g_depth), gx, gshape, gcol, gden, None, ctx.ws, ctx.ws_bytes)
+        return (gx, None, None, None, gshape, gcol, gden.mul_(density_scale)) + (None,) * 10
+
+
 def render_stroke_field(field, coords: torch.Tensor, radius: torch.Tensor, tdist: torch.Tensor,
                         directions: torch.Tensor, bg=1.0, opaque_background: bool = False, no_warp: bool = False,
                         options: Optional[FieldOptions] = None):
@@ -108,13 +177,33 @@ def render_stroke_field(field, coords: torch.Tensor, radius: torch.Tensor, tdist
     if ids is None or ids.device != dev or ids.numel() != S or int(getattr(field, "_n3ds_sdf_id", -1)) != sdf_id:
         ids = torch.full((S,), sdf_id, dtype=torch.int32, device=dev)
         field._n3ds_sdf_ids, field._n3ds_sdf_id = ids, sdf_id
-    window = stroke_window(field)
-    delta = annealed_delta(field, window).expand(S)
-    density = field.density_params * field.density_scale
-    x = warp_coords(getattr(field, "warp_fn", None), coords, float(getattr(field, "bbox_size", 2.0)), no_warp)
-    return render_strokes(x, radius, tdist, directions, field.shape_params, ids, field.color_params, density, delta,
-                          bool(field.use_laplace_transform), bool(field.inv_scale_radius), bg, opaque_background,
-                          options, stroke_window=window)
+    warp_fn, bbox_size = getattr(field, "warp_fn", None), float(getattr(field, "bbox_size", 2.0))
+    if not _plain_state(field, coords, dev):
+        window = stroke_window(field)
+        delta = annealed_delta(field, window).expand(S)
+        density = field.density_params * field.density_scale
+        x = warp_coords(warp_fn, coords, bbox_size, no_warp)
+        return render_strokes(x, radius, tdist, directions, field.shape_params, ids, field.color_params, density,
+                              delta, bool(field.use_laplace_transform), bool(field.inv_scale_radius), bg,
+                              opaque_background, options, stroke_window=window)
+    R = int(coords.shape[0])
+    if coords.dim() != 3 or coords.shape[2] != 3 or radius.shape != coords.shape[:2] or \
+            tdist.shape != (R, coords.shape[1] + 1) or directions.shape != (R, 3):
+        raise ValueError("expected x [R,N,3], radius [R,N], tdist [R,N+1], dirs [R,3]")
+    if field.shape_params.dim() != 2 or field.color_params.shape != (S, 3) or field.density_params.shape != (S,):
+        raise ValueError("expected shape_params [S,P], color_params [S,3], density [S]")
+    # the bbox warp rides along in the state's kernel where no gradient goes back through it
+    scale = None
+    if warp_fn is None and not no_warp and not (coords.requires_grad and torch.is_grad_enabled()):
+        scale = float(np.float32(1.0) / np.float32(bbox_size / 2))  # torch divides by a scalar this way
+        x = coords
+    else:
+        x = warp_coords(warp_fn, coords, bbox_size, no_warp)
+    bg_t, bg_value = (bg, 0.0) if torch.is_tensor(bg) else (None, float(bg))
+    return _ModuleFieldFn.apply(x, radius, tdist, directions, field.shape_params, field.color_params,
+                                field.density_params, bg_t, ids, field.stroke_step, _state_args(field), scale,
+                                bg_value, bool(opaque_background), bool(field.use_laplace_transform),
+                                bool(field.inv_scale_radius), options or FieldOptions())
 
 
 class StrokeField(torch.nn.Module):

@@ -242,3 +242,42 @@ def test_no_host_synchronisation(cuda):
     finally:
         torch.cuda.set_sync_debug_mode(0)
     assert not torch.equal(rgb, rgb2)
+
+
+@pytest.mark.parametrize("training", [True, False])
+@pytest.mark.parametrize("n,step,limit", [(1, 0, None), (255, 1, None), (256, 255, 40), (257, 300, 0), (1000, 617, None)])
+def test_module_inputs_match_the_tensor_expressions(cuda, n, step, limit, training):
+    """The one-launch module state (window, softness, scaled densities, bbox warp) equals
+    the torch expressions it replaces bit for bit, at block edges, and the rendered field
+    with it the field rendered through them (a count of another integer type)."""
+    import ctypes
+    import numpy as np
+    from neural3dstrokes_b200 import _lib
+    from neural3dstrokes_b200 import strokefield as sfm
+    f = StrokeField("sphere", max_num_strokes=n, max_opt_strokes=40, density_scale=17.3, sdf_delta=0.083,
+                    sdf_delta_eval=0.0197, use_laplace_transform=True, bbox_size=3.0, stroke_step_limit=limit).to(cuda)
+    g = torch.Generator().manual_seed(n)
+    sc = scenes.make_strokes(["sphere"] * n, g)
+    with torch.no_grad():
+        f.shape_params.copy_(sc.shape_params[:, :4])
+        f.color_params.copy_(sc.color_params)
+        f.density_params.copy_(torch.rand(n, generator=g))
+        f.stroke_step.fill_(step)
+    f.train(training)
+    x, radius, tdist, dirs = rays_for(cuda, n_rays=7, n_samples=33)
+    window, delta = torch.empty(1, 2, dtype=torch.int32, device=cuda), torch.empty(n, device=cuda)
+    density, warped = torch.empty(n, device=cuda), torch.empty_like(x)
+    max_opt, max_num, has_limit, lim, tr, d0, d1, scale = sfm._state_args(f)
+    m = _lib.ModuleState(_lib.ptr(f.stroke_step), max_opt, max_num, has_limit, lim, tr, d0, d1,
+                         _lib.ptr(f.density_params), scale, float(np.float32(1.0) / np.float32(1.5)))
+    _lib.check(_lib.load().n3ds_field_module_inputs(ctypes.byref(m), n, _lib.ptr(x), x.numel(), _lib.ptr(window),
+                                                    _lib.ptr(delta), _lib.ptr(density), _lib.ptr(warped),
+                                                    _lib.stream_ptr()))
+    want = sfm.stroke_window(f)
+    assert torch.equal(window, want)
+    assert torch.equal(delta, sfm.annealed_delta(f, want).expand(n))
+    assert torch.equal(density, f.density_params * f.density_scale) and torch.equal(warped, x / 1.5)
+    ours = f.render(x, radius, tdist, dirs)
+    f.stroke_step = f.stroke_step.to(torch.int64)  # the torch expressions
+    for a, b in zip(ours, f.render(x, radius, tdist, dirs)):
+        assert torch.equal(a, b)
