@@ -856,18 +856,9 @@ __global__ void ray_bwd_kernel(const RayLaunch L) {
 
 // ============================================================ prep/finalize
 
-__global__ void prep_kernel(const PrepLaunch P) {
-  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (s < P.n_counters) P.counters[s] = 0;
-  if (P.mask_tag && s == 0) *P.mask_tag = P.mask_tag_value;
-  if (P.stats && s < 18) P.stats[s] = 0ull;
-  if (s >= P.n_strokes) return;
-  if (P.gslots) {
-    float* g = P.gslots + s * GRAD_SLOTS;
-#pragma unroll
-    for (int j = 0; j < GRAD_SLOTS; j++) g[j] = 0.f;
-  }
-  float* rec = P.recs + s * REC_FLOATS;
+// One stroke's record (into rec, REC_FLOATS floats of shared memory), culling sphere and
+// margin.
+__device__ void prep_stroke(const PrepLaunch& P, long long s, float* rec) {
   const int wstate = window_state(P.window, P.n_win_scenes, P.win_begin, s);
   if (wstate == 2) {
     // Absent stroke (beyond its scene's active count): a culling sphere of radius
@@ -1104,6 +1095,28 @@ __global__ void prep_kernel(const PrepLaunch P) {
   P.cull_b[s] = plane ? -margin : margin;
 }
 
+// A thread per stroke builds its record in shared memory (odd row pitch: conflict-free),
+// then the block stores the rows, and clears the gradient slots, as consecutive words.
+// Latency bound (a few hundred strokes in a few blocks); with every thread storing its own
+// 256-byte record, cleared first, word by word, 500 strokes took 10.3 us, 4.1 so. It
+// runs before every forward and backward.
+constexpr int PREP_THREADS = 64;
+__global__ void __launch_bounds__(PREP_THREADS) prep_kernel(const PrepLaunch P) {
+  constexpr int PITCH = REC_FLOATS + 1;
+  __shared__ float rows[PREP_THREADS * PITCH];
+  const long long s0 = blockIdx.x * (long long)PREP_THREADS, s = s0 + threadIdx.x;
+  if (s < P.n_counters) P.counters[s] = 0;
+  if (P.mask_tag && s == 0) *P.mask_tag = P.mask_tag_value;
+  if (P.stats && s < 18) P.stats[s] = 0ull;
+  const int n = (int)min((long long)PREP_THREADS, P.n_strokes - s0);  // <= 0: counters only
+  if (P.gslots)
+    for (int i = threadIdx.x; i < n * GRAD_SLOTS; i += PREP_THREADS) P.gslots[s0 * GRAD_SLOTS + i] = 0.f;
+  if (s < P.n_strokes) prep_stroke(P, s, rows + threadIdx.x * PITCH);
+  __syncthreads();
+  for (int i = threadIdx.x; i < n * REC_FLOATS; i += PREP_THREADS)
+    P.recs[s0 * REC_FLOATS + i] = rows[(i / REC_FLOATS) * PITCH + i % REC_FLOATS];
+}
+
 __device__ void prim_param_grads(const FinalizeLaunch& F, long long s, int base, int flags, const float* g,
                                  const float* rec, float* out);
 __device__ void catmull_param_grads(const float* prm, const float* gc, int compat, float* out);
@@ -1305,8 +1318,7 @@ void launch_module_inputs(const ModuleInputs& m, cudaStream_t st) {
 void launch_prep(const PrepLaunch& p, cudaStream_t st) {
   long long n = p.n_strokes > p.n_counters ? p.n_strokes : p.n_counters;
   if (n < 1) n = 1;
-  const int threads = 128;
-  prep_kernel<<<(unsigned)((n + threads - 1) / threads), threads, 0, st>>>(p);
+  prep_kernel<<<(unsigned)((n + PREP_THREADS - 1) / PREP_THREADS), PREP_THREADS, 0, st>>>(p);
 }
 
 template <int W, bool COMMON>
