@@ -108,6 +108,14 @@ int n3ds_compose_backward(float* grad_alphas, float* grad_colors, float* grad_de
                           int64_t n_points, int64_t n_strokes, int64_t color_dim, int grad_mode,
                           void* workspace, size_t workspace_bytes, n3ds_stream_t stream);
 
+/* The same, but grad_alphas and grad_colors are written (they need not be cleared);
+ * grad_density_params still accumulates. */
+int n3ds_compose_backward_write(float* grad_alphas, float* grad_colors, float* grad_density_params,
+                                const float* grad_density_out, const float* grad_color_out, const float* alphas,
+                                const float* colors, const float* density_params, int64_t n_points, int64_t n_strokes,
+                                int64_t color_dim, int grad_mode, void* workspace, size_t workspace_bytes,
+                                n3ds_stream_t stream);
+
 /* Composition modes of compose_strokes other than 'over' (strokes.py:390-417). */
 #define N3DS_COMPOSE_MAX 1
 #define N3DS_COMPOSE_MAX_DENSITY_WEIGHTED 2

@@ -84,6 +84,8 @@ _SIGS = {
     "n3ds_compose_workspace_bytes": (c_size_t, [c_i64, c_i64, ctypes.c_int]),
     "n3ds_compose_backward": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_i64, c_i64, c_i64,
                                              ctypes.c_int, _P, c_size_t, _P]),
+    "n3ds_compose_backward_write": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_i64, c_i64, c_i64,
+                                                   ctypes.c_int, _P, c_size_t, _P]),
     "n3ds_default_options": (None, [ctypes.POINTER(Options)]),
     "n3ds_field_workspace_bytes": (c_size_t, [ctypes.POINTER(Batch), ctypes.POINTER(Options)]),
     "n3ds_field_forward": (ctypes.c_int, [ctypes.POINTER(Batch), ctypes.POINTER(Rays), ctypes.POINTER(Strokes),

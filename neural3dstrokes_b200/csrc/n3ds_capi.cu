@@ -931,11 +931,11 @@ size_t n3ds_compose_workspace_bytes(int64_t n_points, int64_t n_strokes, int gra
   return size_t(n_points) * size_t((n_strokes + 31) / 32) * 4;  // one transmittance per row and 32 strokes
 }
 
-int n3ds_compose_backward(float* grad_alphas, float* grad_colors, float* grad_density_params,
-                          const float* grad_density_out, const float* grad_color_out, const float* alphas,
-                          const float* colors, const float* density_params, int64_t n_points, int64_t n_strokes,
-                          int64_t color_dim, int grad_mode, void* workspace, size_t workspace_bytes,
-                          n3ds_stream_t stream) {
+static int compose_backward(bool write, float* grad_alphas, float* grad_colors, float* grad_density_params,
+                            const float* grad_density_out, const float* grad_color_out, const float* alphas,
+                            const float* colors, const float* density_params, int64_t n_points, int64_t n_strokes,
+                            int64_t color_dim, int grad_mode, void* workspace, size_t workspace_bytes,
+                            n3ds_stream_t stream) {
   if (color_dim != 1 && color_dim != 3)
     return fail(N3DS_ERR_UNSUPPORTED, "Unsupported color dimension: " + std::to_string(color_dim));
   if (n_points < 0 || n_strokes < 0) return fail(N3DS_ERR_INVALID, "negative sizes");
@@ -959,8 +959,29 @@ int n3ds_compose_backward(float* grad_alphas, float* grad_colors, float* grad_de
   L.g_density_params = grad_density_params;
   L.t_scratch = static_cast<float*>(workspace);
   L.compat = compat;
+  L.write_pairs = write;
   N3DS_CUDA_TRY(n3ds::launch_uf_compose_bwd(L, reinterpret_cast<cudaStream_t>(stream)));
   return N3DS_OK;
+}
+
+int n3ds_compose_backward(float* grad_alphas, float* grad_colors, float* grad_density_params,
+                          const float* grad_density_out, const float* grad_color_out, const float* alphas,
+                          const float* colors, const float* density_params, int64_t n_points, int64_t n_strokes,
+                          int64_t color_dim, int grad_mode, void* workspace, size_t workspace_bytes,
+                          n3ds_stream_t stream) {
+  return compose_backward(false, grad_alphas, grad_colors, grad_density_params, grad_density_out, grad_color_out, alphas,
+                          colors, density_params, n_points, n_strokes, color_dim, grad_mode, workspace,
+                          workspace_bytes, stream);
+}
+
+int n3ds_compose_backward_write(float* grad_alphas, float* grad_colors, float* grad_density_params,
+                                const float* grad_density_out, const float* grad_color_out, const float* alphas,
+                                const float* colors, const float* density_params, int64_t n_points, int64_t n_strokes,
+                                int64_t color_dim, int grad_mode, void* workspace, size_t workspace_bytes,
+                                n3ds_stream_t stream) {
+  return compose_backward(true, grad_alphas, grad_colors, grad_density_params, grad_density_out, grad_color_out, alphas,
+                          colors, density_params, n_points, n_strokes, color_dim, grad_mode, workspace,
+                          workspace_bytes, stream);
 }
 
 // ---------------------------------------------------------------------- Adam

@@ -4,9 +4,8 @@
 //                 (local) sample on the segment pos0 -> pos1 (12 parameters);
 //   SH2 / SH3     sigmoid(sum_i coef_i Y_i(viewdir)) per channel, real spherical
 //                 harmonics of the world view direction (12 / 27 parameters).
-// Lane = stroke (32 strokes per warp tile) and a loop over samples, so the colour rows
-// are written and read coalesced and each lane keeps its stroke's parameters and
-// parameter gradients in registers. The backward accumulates the colour-parameter
+// Lane = stroke (32 strokes per warp tile) and a loop over samples: each lane keeps its
+// stroke's parameters and parameter gradients in registers. The backward accumulates the colour-parameter
 // gradients (the reference's formulas, exact in the parameters) and, in exact mode,
 // the gradient rgb's dependence on the sample position, which it sends through the
 // stroke transform into the reduced slots and grad_x (the reference drops that term).
@@ -41,12 +40,6 @@ __device__ __forceinline__ void sh_basis(V3 d, float (&w)[N]) {
     w[8] = c22 * (d.x * d.x - d.y * d.y);
   }
 }
-
-template <int CT>
-struct ColorDims {
-  static constexpr int NP = CT == 3 ? 27 : 12;  // colour parameters
-  static constexpr int NB = CT == 3 ? 9 : 4;    // SH terms
-};
 
 // Local (unit-frame) sample of the stroke: the primitives' inverse transform; the
 // curves have none.
@@ -90,43 +83,27 @@ __device__ __forceinline__ V3 transform_backprop(const float* rec, int kind, V3 
   return xyz(rec4(rec)[R_M / 4]) * gp.x + xyz(rec4(rec)[R_M / 4 + 1]) * gp.y + xyz(rec4(rec)[R_M / 4 + 2]) * gp.z;
 }
 
-template <int CT>
-__global__ void __launch_bounds__(COL_WARPS * 32) uf_color_fwd_kernel(const UfColor L) {
-  constexpr int NP = ColorDims<CT>::NP;
+__global__ void __launch_bounds__(COL_WARPS * 32) uf_gradient_rgb_fwd_kernel(const UfColor L) {
   __shared__ __align__(16) float recs[32 * COL_RS];
   const int s0 = blockIdx.y * 32;
   const int ns = min(32, L.n_strokes - s0);
-  if (CT == 1)
-    for (int i = threadIdx.x; i < ns * REC_FLOATS; i += blockDim.x)
-      recs[(i / REC_FLOATS) * COL_RS + (i % REC_FLOATS)] = L.recs[(long long)s0 * REC_FLOATS + i];
+  for (int i = threadIdx.x; i < ns * REC_FLOATS; i += blockDim.x)
+    recs[(i / REC_FLOATS) * COL_RS + (i % REC_FLOATS)] = L.recs[(long long)s0 * REC_FLOATS + i];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool active = lane < ns;
   const long long s = s0 + (active ? lane : 0);
   const float* rec = recs + (active ? lane : 0) * COL_RS;
-  const int kind = CT == 1 ? __float_as_int(rec[R_KIND]) : 0;
-  float cp[NP];
+  const int kind = __float_as_int(rec[R_KIND]);
+  float cp[12];
 #pragma unroll
-  for (int k = 0; k < NP; k++) cp[k] = L.color_params[s * L.color_stride + k];
+  for (int k = 0; k < 12; k++) cp[k] = L.color_params[s * L.color_stride + k];
   const long long S = L.n_strokes;
   for (long long p = (long long)blockIdx.x * COL_WARPS + warp; p < L.n_points; p += (long long)gridDim.x * COL_WARPS) {
-    V3 c;
-    if constexpr (CT == 1) {
-      const V3 x = v3(L.x[3 * p], L.x[3 * p + 1], L.x[3 * p + 2]);
-      float t, d0, d1;
-      V3 v0, v1;
-      c = gradient_rgb(cp, unit_pos(rec, kind & 15, x), &t, &d0, &d1, &v0, &v1);
-    } else {
-      const long long r = p / L.spr;
-      float w[ColorDims<CT>::NB];
-      sh_basis(v3(L.viewdir[3 * r], L.viewdir[3 * r + 1], L.viewdir[3 * r + 2]), w);
-      float acc[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < ColorDims<CT>::NB; i++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) acc[q] += cp[3 * i + q] * w[i];
-      c = v3(sigmoidf_(acc[0]), sigmoidf_(acc[1]), sigmoidf_(acc[2]));
-    }
+    const V3 x = v3(L.x[3 * p], L.x[3 * p + 1], L.x[3 * p + 2]);
+    float t, d0, d1;
+    V3 v0, v1;
+    const V3 c = gradient_rgb(cp, unit_pos(rec, kind & 15, x), &t, &d0, &d1, &v0, &v1);
     if (active) {
       float* o = L.color + (p * S + s) * 3;
       o[0] = c.x;
@@ -136,89 +113,63 @@ __global__ void __launch_bounds__(COL_WARPS * 32) uf_color_fwd_kernel(const UfCo
   }
 }
 
-template <int CT>
-__global__ void __launch_bounds__(COL_WARPS * 32) uf_color_bwd_kernel(const UfColor L) {
-  constexpr int NP = ColorDims<CT>::NP;
+__global__ void __launch_bounds__(COL_WARPS * 32) uf_gradient_rgb_bwd_kernel(const UfColor L) {
   __shared__ __align__(16) float recs[32 * COL_RS];
   const int s0 = blockIdx.y * 32;
   const int ns = min(32, L.n_strokes - s0);
-  if (CT == 1)
-    for (int i = threadIdx.x; i < ns * REC_FLOATS; i += blockDim.x)
-      recs[(i / REC_FLOATS) * COL_RS + (i % REC_FLOATS)] = L.recs[(long long)s0 * REC_FLOATS + i];
+  for (int i = threadIdx.x; i < ns * REC_FLOATS; i += blockDim.x)
+    recs[(i / REC_FLOATS) * COL_RS + (i % REC_FLOATS)] = L.recs[(long long)s0 * REC_FLOATS + i];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool active = lane < ns;
   const long long s = s0 + (active ? lane : 0);
   const float* rec = recs + (active ? lane : 0) * COL_RS;
-  const int kind = CT == 1 ? __float_as_int(rec[R_KIND]) : 0;
+  const int kind = __float_as_int(rec[R_KIND]);
   const int base = kind & 15;
-  float cp[NP], gcp[NP];
+  float cp[12], gcp[12];
 #pragma unroll
-  for (int k = 0; k < NP; k++) {
+  for (int k = 0; k < 12; k++) {
     cp[k] = L.color_params[s * L.color_stride + k];
     gcp[k] = 0.f;
   }
   float v[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // GP, torque, scale slots
-  const bool with_pos = CT == 1 && !L.compat;
+  const bool with_pos = !L.compat;
   const long long S = L.n_strokes;
   for (long long p = (long long)blockIdx.x * COL_WARPS + warp; p < L.n_points; p += (long long)gridDim.x * COL_WARPS) {
     const float* gcol = L.g_color + (p * S + s) * 3;
     const V3 g = active ? v3(gcol[0], gcol[1], gcol[2]) : v3(0.f, 0.f, 0.f);
-    if constexpr (CT == 1) {
-      const V3 x = v3(L.x[3 * p], L.x[3 * p + 1], L.x[3 * p + 2]);
-      const V3 pl = unit_pos(rec, base, x);
-      float t, d0, d1;
-      V3 v0, v1;
-      gradient_rgb(cp, pl, &t, &d0, &d1, &v0, &v1);
-      // strokes_color.h:82-96
-      const float gt = dot(g, v3(cp[9] - cp[6], cp[10] - cp[7], cp[11] - cp[8]));
-      const float gtr = 5.0f * t * (1.0f - t) * gt;
-      const float gd0 = gtr / d1, gd1 = -gtr * d0 / (d1 * d1);
-      const V3 gv1 = v0 * gd0 + v1 * (gd1 * 2.0f);
-      const V3 gv0 = v1 * gd0;
-      const V3 gp0 = -gv0 - gv1;
-      gcp[0] += gp0.x; gcp[1] += gp0.y; gcp[2] += gp0.z;
-      gcp[3] += gv1.x; gcp[4] += gv1.y; gcp[5] += gv1.z;
-      gcp[6] += g.x * (1.0f - t); gcp[7] += g.y * (1.0f - t); gcp[8] += g.z * (1.0f - t);
-      gcp[9] += g.x * t; gcp[10] += g.y * t; gcp[11] += g.z * t;
-      if (with_pos) {
-        // dL/d(local p) = dL/dv0 = gd0 v1
-        const V3 gx = base <= B_TETRAHEDRON ? transform_backprop(rec, kind, pl, gv0, v) : gv0;
-        if (L.grad_x) {
-          const float sx = warp_sum(gx.x), sy = warp_sum(gx.y), sz = warp_sum(gx.z);
-          if (lane == 0) {
-            atomicAdd(L.grad_x + 3 * p, sx);
-            atomicAdd(L.grad_x + 3 * p + 1, sy);
-            atomicAdd(L.grad_x + 3 * p + 2, sz);
-          }
+    const V3 x = v3(L.x[3 * p], L.x[3 * p + 1], L.x[3 * p + 2]);
+    const V3 pl = unit_pos(rec, base, x);
+    float t, d0, d1;
+    V3 v0, v1;
+    gradient_rgb(cp, pl, &t, &d0, &d1, &v0, &v1);
+    // strokes_color.h:82-96
+    const float gt = dot(g, v3(cp[9] - cp[6], cp[10] - cp[7], cp[11] - cp[8]));
+    const float gtr = 5.0f * t * (1.0f - t) * gt;
+    const float gd0 = gtr / d1, gd1 = -gtr * d0 / (d1 * d1);
+    const V3 gv1 = v0 * gd0 + v1 * (gd1 * 2.0f);
+    const V3 gv0 = v1 * gd0;
+    const V3 gp0 = -gv0 - gv1;
+    gcp[0] += gp0.x; gcp[1] += gp0.y; gcp[2] += gp0.z;
+    gcp[3] += gv1.x; gcp[4] += gv1.y; gcp[5] += gv1.z;
+    gcp[6] += g.x * (1.0f - t); gcp[7] += g.y * (1.0f - t); gcp[8] += g.z * (1.0f - t);
+    gcp[9] += g.x * t; gcp[10] += g.y * t; gcp[11] += g.z * t;
+    if (with_pos) {
+      // dL/d(local p) = dL/dv0 = gd0 v1
+      const V3 gx = base <= B_TETRAHEDRON ? transform_backprop(rec, kind, pl, gv0, v) : gv0;
+      if (L.grad_x) {
+        const float sx = warp_sum(gx.x), sy = warp_sum(gx.y), sz = warp_sum(gx.z);
+        if (lane == 0) {
+          atomicAdd(L.grad_x + 3 * p, sx);
+          atomicAdd(L.grad_x + 3 * p + 1, sy);
+          atomicAdd(L.grad_x + 3 * p + 2, sz);
         }
       }
-    } else {
-      const long long r = p / L.spr;
-      constexpr int NB = ColorDims<CT>::NB;
-      float w[NB];
-      sh_basis(v3(L.viewdir[3 * r], L.viewdir[3 * r + 1], L.viewdir[3 * r + 2]), w);
-      float acc[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < NB; i++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) acc[q] += cp[3 * i + q] * w[i];
-      float gr[3];
-      const float gq[3] = {g.x, g.y, g.z};
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        const float c = sigmoidf_(acc[q]);
-        gr[q] = gq[q] * c * (1.0f - c);
-      }
-#pragma unroll
-      for (int i = 0; i < NB; i++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) gcp[3 * i + q] += gr[q] * w[i];
     }
   }
   if (active) {
 #pragma unroll
-    for (int k = 0; k < NP; k++)
+    for (int k = 0; k < 12; k++)
       if (gcp[k] != 0.f) atomicAdd(L.grad_color_params + s * L.color_stride + k, gcp[k]);
     if (with_pos && base <= B_TETRAHEDRON) {
       float* row = L.gslots + s * GRAD_SLOTS;
@@ -229,6 +180,87 @@ __global__ void __launch_bounds__(COL_WARPS * 32) uf_color_bwd_kernel(const UfCo
         if (v[6 + k] != 0.f) atomicAdd(row + G_SCALE + k, v[6 + k]);
       }
     }
+  }
+}
+
+// SH colours: constant along a ray, so a warp takes up to SH_PIECE consecutive samples of
+// one view direction at a time, evaluates the field once and streams the colour rows. A row
+// of the 32-stroke block is 96 consecutive floats: element lane + 32 k of it belongs to
+// stroke e / 3, channel e % 3, so three coalesced accesses move it; the backward sums
+// the upstream rows by element and takes its own stroke's sums once per piece. HBM bound
+// (12 B per pair): 19,904 samples x 131 strokes, SH3: forward 19 -> 9 us, backward 115
+// -> 36 us (the harmonics, sigmoid and 27 parameter gradients per sample and stroke before).
+constexpr int SH_PIECE = 16;
+
+__device__ __forceinline__ float sel3(int q, float a, float b, float c) { return q == 0 ? a : (q == 1 ? b : c); }
+
+template <int CT, bool BWD>
+__global__ void __launch_bounds__(COL_WARPS * 32) uf_sh_kernel(const UfColor L) {
+  constexpr int NB = CT == 3 ? 9 : 4, NP = 3 * NB;
+  const int s0 = blockIdx.y * 32;
+  const int ns = min(32, L.n_strokes - s0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool active = lane < ns;
+  const long long s = s0 + (active ? lane : 0);
+  float cp[NP], gcp[BWD ? NP : 1];
+#pragma unroll
+  for (int k = 0; k < NP; k++) {
+    cp[k] = L.color_params[s * L.color_stride + k];
+    if (BWD) gcp[k] = 0.f;
+  }
+  const long long S3 = 3LL * L.n_strokes;
+  const long long ppr = (L.spr + SH_PIECE - 1) / SH_PIECE;  // pieces per view direction
+  const long long pieces = (L.n_points / L.spr) * ppr;
+  for (long long i = (long long)blockIdx.x * COL_WARPS + warp; i < pieces; i += (long long)gridDim.x * COL_WARPS) {
+    const long long r = i / ppr;
+    const long long k0 = (i - r * ppr) * SH_PIECE;
+    const int n = (int)min((long long)SH_PIECE, L.spr - k0);
+    const long long row = (r * L.spr + k0) * S3 + 3LL * s0 + lane;  // element `lane` of the first row
+    float w[NB];
+    sh_basis(v3(L.viewdir[3 * r], L.viewdir[3 * r + 1], L.viewdir[3 * r + 2]), w);
+    float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+#pragma unroll
+      for (int q = 0; q < 3; q++) acc[q] += cp[3 * b + q] * w[b];
+    const float c[3] = {sigmoidf_(acc[0]), sigmoidf_(acc[1]), sigmoidf_(acc[2])};
+    if constexpr (!BWD) {
+      float e[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        const int el = lane + 32 * k, src = el / 3, q = el - 3 * src;
+        const float a0 = __shfl_sync(0xffffffffu, c[0], src), a1 = __shfl_sync(0xffffffffu, c[1], src),
+                    a2 = __shfl_sync(0xffffffffu, c[2], src);
+        e[k] = sel3(q, a0, a1, a2);
+      }
+      for (int j = 0; j < n; j++) {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          if (lane + 32 * k < 3 * ns) L.color[row + j * S3 + 32 * k] = e[k];
+      }
+    } else {
+      float e[3] = {0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int j = 0; j < n; j++) {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          if (lane + 32 * k < 3 * ns) e[k] += __ldg(L.g_color + row + j * S3 + 32 * k);
+      }
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        const int el = 3 * lane + q, src = el & 31, k = el >> 5;
+        const float a0 = __shfl_sync(0xffffffffu, e[0], src), a1 = __shfl_sync(0xffffffffu, e[1], src),
+                    a2 = __shfl_sync(0xffffffffu, e[2], src);
+        const float gr = sel3(k, a0, a1, a2) * c[q] * (1.0f - c[q]);
+#pragma unroll
+        for (int b = 0; b < NB; b++) gcp[3 * b + q] += gr * w[b];
+      }
+    }
+  }
+  if (BWD && active) {
+#pragma unroll
+    for (int k = 0; k < NP; k++)
+      if (gcp[k] != 0.f) atomicAdd(L.grad_color_params + s * L.color_stride + k, gcp[k]);
   }
 }
 
@@ -302,23 +334,28 @@ __global__ void __launch_bounds__(COL_WARPS * 32) uf_texcoord_kernel(const UfCol
   }
 }
 
-// one wave of the kernel's resident blocks over the stroke blocks
+// one wave of the kernel's resident blocks over the stroke blocks, at most one warp per item
 template <typename K>
-cudaError_t color_grid(const UfColor& L, K kernel, dim3* grid) {
+cudaError_t color_grid(const UfColor& L, K kernel, dim3* grid, long long items) {
   const int sblocks = (L.n_strokes + 31) / 32;
   long long want = 1;
-  cudaError_t e = one_wave_blocks(kernel, COL_WARPS * 32, sblocks, (L.n_points + COL_WARPS - 1) / COL_WARPS, &want);
+  cudaError_t e = one_wave_blocks(kernel, COL_WARPS * 32, sblocks, (items + COL_WARPS - 1) / COL_WARPS, &want);
   *grid = dim3((unsigned)want, sblocks);
   return e;
+}
+
+// Work items of a warp: samples, or pieces of a view direction's samples (SH).
+long long color_items(const UfColor& L) {
+  return L.color_id == 1 ? L.n_points : (L.n_points / L.spr) * ((L.spr + SH_PIECE - 1) / SH_PIECE);
 }
 
 }  // namespace
 
 cudaError_t launch_uf_color_fwd(const UfColor& L, cudaStream_t st) {
   if (L.color_id < 1 || L.color_id > 3) return cudaErrorInvalidValue;
-  auto* k = L.color_id == 1 ? uf_color_fwd_kernel<1> : L.color_id == 2 ? uf_color_fwd_kernel<2> : uf_color_fwd_kernel<3>;
+  auto* k = L.color_id == 1 ? uf_gradient_rgb_fwd_kernel : L.color_id == 2 ? uf_sh_kernel<2, false> : uf_sh_kernel<3, false>;
   dim3 grid;
-  cudaError_t e = color_grid(L, k, &grid);
+  cudaError_t e = color_grid(L, k, &grid, color_items(L));
   if (e != cudaSuccess) return e;
   k<<<grid, COL_WARPS * 32, 0, st>>>(L);
   return cudaGetLastError();
@@ -326,7 +363,7 @@ cudaError_t launch_uf_color_fwd(const UfColor& L, cudaStream_t st) {
 
 cudaError_t launch_uf_texcoord(const UfColor& L, float* texcoord, cudaStream_t st) {
   dim3 grid;
-  cudaError_t e = color_grid(L, uf_texcoord_kernel, &grid);
+  cudaError_t e = color_grid(L, uf_texcoord_kernel, &grid, L.n_points);
   if (e != cudaSuccess) return e;
   uf_texcoord_kernel<<<grid, COL_WARPS * 32, 0, st>>>(L, texcoord);
   return cudaGetLastError();
@@ -334,9 +371,9 @@ cudaError_t launch_uf_texcoord(const UfColor& L, float* texcoord, cudaStream_t s
 
 cudaError_t launch_uf_color_bwd(const UfColor& L, cudaStream_t st) {
   if (L.color_id < 1 || L.color_id > 3) return cudaErrorInvalidValue;
-  auto* k = L.color_id == 1 ? uf_color_bwd_kernel<1> : L.color_id == 2 ? uf_color_bwd_kernel<2> : uf_color_bwd_kernel<3>;
+  auto* k = L.color_id == 1 ? uf_gradient_rgb_bwd_kernel : L.color_id == 2 ? uf_sh_kernel<2, true> : uf_sh_kernel<3, true>;
   dim3 grid;
-  cudaError_t e = color_grid(L, k, &grid);
+  cudaError_t e = color_grid(L, k, &grid, color_items(L));
   if (e != cudaSuccess) return e;
   k<<<grid, COL_WARPS * 32, 0, st>>>(L);
   return cudaGetLastError();

@@ -188,10 +188,10 @@ __global__ void __launch_bounds__(UF_WARPS * 32) uf_stroke_bwd_kernel(const UfSt
   // recompute and adjoint, so their latency overlaps the work: without it each
   // iteration's loads wait behind the previous iteration's grad_x atomics.
   struct In {
-    float x0, x1, x2, r, ga, a, gs, gc0, gc1, gc2;
+    float x0, x1, x2, r, ga, a, gs;
   };
   auto fetch = [&](long long q, In& in) {
-    in = In{0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    in = In{0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f};
     if (q >= L.n_points) return;
     in.x0 = __ldg(L.x + 3 * q);
     in.x1 = __ldg(L.x + 3 * q + 1);
@@ -202,35 +202,40 @@ __global__ void __launch_bounds__(UF_WARPS * 32) uf_stroke_bwd_kernel(const UfSt
     in.ga = __ldg(L.g_alpha + qi);
     in.a = __ldg(L.alpha_in + qi);
     if (L.g_sdf) in.gs = __ldg(L.g_sdf + qi);
-    if (L.color_const) {
-      in.gc0 = __ldg(L.g_color + 3 * qi);
-      in.gc1 = __ldg(L.g_color + 3 * qi + 1);
-      in.gc2 = __ldg(L.g_color + 3 * qi + 2);
-    }
+  };
+  // Upstream colour rows of the 32-stroke block by element (lane + 32 k of 96: stroke e / 3,
+  // channel e % 3), three coalesced loads a sample; summed over all samples by element, the
+  // lane's own stroke is picked at the end.
+  auto fetch_color = [&](long long q, float (&e)[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      e[k] = q < L.n_points && lane + 32 * k < 3 * ns ? __ldg(L.g_color + (q * S + s0) * 3 + lane + 32 * k) : 0.f;
   };
   const long long pstep = (long long)gridDim.x * UF_WARPS;
   long long p = (long long)blockIdx.x * UF_WARPS + warp;
   In cur;
   fetch(p, cur);
+  float ecur[3] = {0.f, 0.f, 0.f}, esum[3] = {0.f, 0.f, 0.f};
+  if (L.color_const) fetch_color(p, ecur);
   for (; p < L.n_points; p += pstep) {
     In nxt;
     fetch(p + pstep, nxt);
+    float enxt[3] = {0.f, 0.f, 0.f};
+    if (L.color_const) fetch_color(p + pstep, enxt);
     const V3 x = v3(cur.x0, cur.x1, cur.x2);
     const float rinv = 1.f / cur.r;
     const float ga = cur.ga, a = cur.a, gs = cur.gs;
-    if (active && L.color_const) {
-      v[G_COLOR] += cur.gc0;
-      v[G_COLOR + 1] += cur.gc1;
-      v[G_COLOR + 2] += cur.gc2;
-    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) esum[k] += ecur[k];
 
     float sdf, f = 1.f;
-    V3 pl;
+    V3 pl, gsdf;
+    float gbp[2];
     QuadFwd qf;
     CubicFwd cf;
     if (CLS == UF_PRIM) {
       pl = prim_local(rec, x);
-      sdf = prim_sdf(base, pl, rec);
+      sdf = compat ? prim_sdf(base, pl, rec) : prim_sdf_grad(base, pl, rec, &gsdf, gbp);
       if (kind & K_S3FAC) f = s3_factor(base, pl, xyz(rec4(rec)[R_S / 4]), rec);
     } else if (CLS == UF_QUAD) {
       sdf = quad_eval(rec, x, qf);
@@ -257,7 +262,8 @@ __global__ void __launch_bounds__(UF_WARPS * 32) uf_stroke_bwd_kernel(const UfSt
     v[G_K] += K;
     V3 gx;
     if (CLS == UF_PRIM) {
-      gx = prim_backprop(rec, kind, pl, dsdf, K, v, compat);
+      gx = compat ? prim_backprop(rec, kind, pl, dsdf, K, v, compat)
+                  : prim_backprop(rec, kind, pl, dsdf, K, v, 0, gsdf, gbp);
     } else if (CLS == UF_QUAD) {
       gx = quad_adjoint(rec, qf, dsdf, v + G_CTRL);
     } else {
@@ -273,6 +279,17 @@ __global__ void __launch_bounds__(UF_WARPS * 32) uf_stroke_bwd_kernel(const UfSt
       }
     }
     cur = nxt;
+#pragma unroll
+    for (int k = 0; k < 3; k++) ecur[k] = enxt[k];
+  }
+  if (L.color_const) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const int el = 3 * lane + q, src = el & 31, k = el >> 5;
+      const float a0 = __shfl_sync(0xffffffffu, esum[0], src), a1 = __shfl_sync(0xffffffffu, esum[1], src),
+                  a2 = __shfl_sync(0xffffffffu, esum[2], src);
+      v[G_COLOR + q] += k == 0 ? a0 : (k == 1 ? a1 : a2);
+    }
   }
   if (active) {
     float* dst = L.gslots + (long long)(s0 + lane) * GRAD_SLOTS;
@@ -327,6 +344,12 @@ __device__ __forceinline__ void load_tile(ComposeTiles<C, W>& t, int warp, int l
 // coalesced row segments, nothing is staged: the kernel streams alphas and colours
 // once (16 B per pair for C = 3).
 constexpr int UCR_WARPS = 8;  // row kernels: warps per block
+
+// A per-pair gradient, accumulated into the caller's buffer or (write_pairs) stored: every
+// backward kernel visits each pair once, so a caller with fresh buffers saves clearing
+// them and reading them back (16 of 48 bytes a pair, and the fill's 16: 65,536 x 256, 155 ->
+// 117 us and 42 -> 4 us of fills).
+__device__ __forceinline__ void put_pair(const UfCompose& L, float* dst, float v) { *dst = L.write_pairs ? v : *dst + v; }
 
 __device__ __forceinline__ float excl_prod_up(float v, int lane) {
   // exclusive product over lanes below (lower index); lane 0 gets 1
@@ -583,9 +606,9 @@ __global__ void __launch_bounds__(UCR_WARPS * 32) uf_compose_bwd_rows(const UfCo
       for (int ch = 0; ch < C; ch++) inner += gC[ch] * (c[ch] - fmaf(em, cV[ch], eV[ch]));
       if (in) {
         const float w = a * Ts;
-        L.g_alphas[p * S + s] += Ts * inner;
+        put_pair(L, L.g_alphas + p * S + s, Ts * inner);
 #pragma unroll
-        for (int ch = 0; ch < C; ch++) L.g_colors[(p * S + s) * C + ch] += gC[ch] * w;
+        for (int ch = 0; ch < C; ch++) put_pair(L, L.g_colors + (p * S + s) * C + ch, gC[ch] * w);
         if (L.g_density_params) {
           const float g = gd * w;
           if (g != 0.0f) {
@@ -633,6 +656,7 @@ __global__ void __launch_bounds__(UCR_WARPS * 32) uf_compose_bwd_vec(const UfCom
 #pragma unroll
   for (int j = 0; j < NJ; j++) gdp_reg[j] = 0.0f;
   const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool write = L.write_pairs != 0;
   for (long long p = (long long)blockIdx.x * UCR_WARPS + (threadIdx.x >> 5); p < L.n_points;
        p += (long long)gridDim.x * UCR_WARPS) {
     const float4* __restrict__ arow = reinterpret_cast<const float4*>(L.alphas + p * S);
@@ -801,12 +825,12 @@ __global__ void __launch_bounds__(UCR_WARPS * 32) uf_compose_bwd_vec(const UfCom
 #pragma unroll
       for (int i = 0; i < G; i++) {
         if ((gq + i) * 4 < S) {
-          float4 v = garow[gq + i];
+          float4 v = write ? z4 : garow[gq + i];
           v.x += ga[4 * i]; v.y += ga[4 * i + 1]; v.z += ga[4 * i + 2]; v.w += ga[4 * i + 3];
           garow[gq + i] = v;
 #pragma unroll
           for (int h = 0; h < C; h++) {
-            float4 u = gcrow[(gq + i) * C + h];
+            float4 u = write ? z4 : gcrow[(gq + i) * C + h];
             u.x += gcc[4 * C * i + 4 * h]; u.y += gcc[4 * C * i + 4 * h + 1];
             u.z += gcc[4 * C * i + 4 * h + 2]; u.w += gcc[4 * C * i + 4 * h + 3];
             gcrow[(gq + i) * C + h] = u;
@@ -936,10 +960,10 @@ __global__ void __launch_bounds__(UCB_WARPS * 32) uf_compose_bwd_kernel(const Uf
         __syncwarp();
         for (int rr = 0; rr < rows; rr++) {
           const long long row = (p0 + rr) * SS;
-          if (lane < nb) L.g_alphas[row + hi - lane] += tx[warp][rr][lane];
+          if (lane < nb) put_pair(L, L.g_alphas + row + hi - lane, tx[warp][rr][lane]);
           for (int e = lane; e < nb * C; e += 32) {
             const int j = e / C, ch = e - j * C;
-            L.g_colors[(row + hi - j) * C + ch] += tg[warp][rr][j * C + ch];
+            put_pair(L, L.g_colors + (row + hi - j) * C + ch, tg[warp][rr][j * C + ch]);
           }
         }
         if (lane < nb) {
@@ -986,10 +1010,10 @@ __global__ void __launch_bounds__(UCB_WARPS * 32) uf_compose_bwd_kernel(const Uf
         __syncwarp();
         for (int rr = 0; rr < rows; rr++) {
           const long long row = (p0 + rr) * SS;
-          if (lane < nb) L.g_alphas[row + lo + lane] += tx[warp][rr][lane];
+          if (lane < nb) put_pair(L, L.g_alphas + row + lo + lane, tx[warp][rr][lane]);
           for (int e = lane; e < nb * C; e += 32) {
             const int j = e / C, ch = e - j * C;
-            L.g_colors[(row + lo + j) * C + ch] += tg[warp][rr][j * C + ch];
+            put_pair(L, L.g_colors + (row + lo + j) * C + ch, tg[warp][rr][j * C + ch]);
           }
         }
         if (lane < nb) {

@@ -69,6 +69,7 @@ struct UfCompose {
   float* g_density_params; // [S] accumulated
   float* t_scratch;        // [P*S] exact mode only
   int compat;
+  int write_pairs;         // backward: store g_alphas and g_colors instead of accumulating into them
 };
 
 // Blocks per 32-stroke block for a kernel whose warps stride over the samples: one wave

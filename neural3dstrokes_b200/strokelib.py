@@ -135,6 +135,14 @@ def compose_forward(density_output, color_output, alphas, colors, density_params
 def compose_backward(grad_alphas, grad_colors, grad_density_params, grad_density_output, grad_color_output,
                      alphas, colors, density_params):
     """compositing.cu:206-262: accumulates grad_alphas, grad_colors, grad_density_params."""
+    _compose_backward("n3ds_compose_backward", grad_alphas, grad_colors, grad_density_params, grad_density_output,
+                      grad_color_output, alphas, colors, density_params)
+
+
+def _compose_backward(entry, grad_alphas, grad_colors, grad_density_params, grad_density_output, grad_color_output,
+                      alphas, colors, density_params):
+    """``entry``: n3ds_compose_backward, or n3ds_compose_backward_write, which stores
+    grad_alphas and grad_colors instead of adding to them."""
     for n, t in zip(["grad_alphas", "grad_colors", "grad_density_params", "grad_density_output",
                      "grad_color_output", "alphas", "colors", "density_params"],
                     [grad_alphas, grad_colors, grad_density_params, grad_density_output, grad_color_output,
@@ -150,7 +158,7 @@ def compose_backward(grad_alphas, grad_colors, grad_density_params, grad_density
     with torch.cuda.device(alphas.device):
         ws_bytes = lib.n3ds_compose_workspace_bytes(P, S, _grad_mode)
         ws = _lib.workspace(ws_bytes, alphas.device) if ws_bytes else None
-        rc = lib.n3ds_compose_backward(
+        rc = getattr(lib, entry)(
             _lib.ptr(grad_alphas), _lib.ptr(grad_colors), _lib.ptr(grad_density_params),
             _lib.ptr(grad_density_output), _lib.ptr(grad_color_output), _lib.ptr(alphas), _lib.ptr(colors),
             _lib.ptr(density_params), P, S, C, _grad_mode, _lib.ptr(ws), ws_bytes, _lib.stream_ptr())

@@ -227,8 +227,8 @@ class _ComposeFn(torch.autograd.Function):
         dev = a.device
         gd = torch.zeros(0, device=dev) if g_dens is None else g_dens.contiguous().float().reshape(-1)
         gc = torch.zeros(0, device=dev) if g_col is None else g_col.contiguous().float().reshape(-1, c.shape[-1])
-        ga, gcs, gdp = torch.zeros_like(a), torch.zeros_like(c), torch.zeros_like(d)
-        _backend.compose_backward(ga, gcs, gdp, gd, gc, a, c, d)
+        ga, gcs, gdp = torch.empty_like(a), torch.empty_like(c), torch.zeros_like(d)
+        _backend._compose_backward("n3ds_compose_backward_write", ga, gcs, gdp, gd, gc, a, c, d)
         S = d.shape[0]
         return ga.reshape(*ctx.pre, S), gcs.reshape(*ctx.pre, S, c.shape[-1]), gdp
 

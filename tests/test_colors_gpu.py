@@ -125,3 +125,28 @@ def test_texcoord_matches_oracle(cuda, kind):
     d = (tex.cpu().double() - tex_r).abs()
     d = torch.minimum(d, (1.0 - d).abs())
     assert float(d.max()) < 1e-5, float(d.max())
+
+
+@pytest.mark.parametrize("color_id", [2, 3])
+@pytest.mark.parametrize("spr,S", [(1, 1), (15, 31), (16, 32), (17, 33), (40, 70)])
+def test_sh_pieces_match_float64(cuda, color_id, spr, S):
+    """The SH colours and their parameter gradients, taken in pieces of a ray's samples, at
+    the edges of a piece and of a 32-stroke block. Tolerances: 1e-5 and 1e-4."""
+    from neural3dstrokes_b200 import strokes as st_api
+    from oracle import strokefield as osf
+    R, n = 5, 12 if color_id == 2 else 27
+    g = torch.Generator().manual_seed(100 * spr + S)
+    fn = st_api.get_stroke("sphere", "constant_sh2" if color_id == 2 else "constant_sh3", "recon")[0]
+    x = torch.rand(R, spr, 3, generator=g) * 2 - 1
+    dirs = torch.nn.functional.normalize(torch.randn(R, 3, generator=g), dim=-1)
+    shape = torch.cat([torch.rand(S, 1, generator=g) * 0.3 + 0.1, torch.rand(S, 3, generator=g) * 2 - 1], 1)
+    col = torch.randn(S, n, generator=g)
+    up = torch.randn(R, spr, S, 3, generator=g)
+    c = col.to(cuda).requires_grad_(True)
+    _, color, _, _ = fn(x.to(cuda), torch.ones(R, spr, device=cuda), dirs.to(cuda), shape.to(cuda), c, 0.1, True, True)
+    got, = torch.autograd.grad(color, c, up.to(cuda))
+    c64 = col.double().requires_grad_(True)
+    w = osf.sh_weights(color_id, dirs.double())
+    want = torch.sigmoid(torch.einsum("rn,snc->rsc", w, c64.reshape(S, n // 3, 3)))[:, None].expand(R, spr, S, 3)
+    ref, = torch.autograd.grad(want, c64, up.double())
+    assert rel(color, want) < 1e-5 and rel(got, ref) < 1e-4

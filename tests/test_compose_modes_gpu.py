@@ -47,3 +47,47 @@ def test_unknown_mode_raises(cuda):
     with pytest.raises(ValueError):
         compose_strokes(torch.rand(2, 3, device=cuda), torch.rand(2, 3, 3, device=cuda), torch.rand(3, device=cuda),
                         "median")
+
+
+@pytest.mark.parametrize("S", [1, 31, 32, 33, 64, 65, 128, 129, 192, 193, 256, 257])
+@pytest.mark.parametrize("mode", ["softmax", "softmax_density_weighted"])
+def test_softmax_modes_at_register_edges(cuda, mode, S):
+    """Forward and gradients against float64 at the stroke counts where the register
+    kernels change (257: the general one). Tolerances: 1e-5 and 1e-4."""
+    from neural3dstrokes_b200 import strokes as st_api
+    g = torch.Generator().manual_seed(S)
+    a, c, d = torch.rand(37, S, generator=g), torch.rand(37, S, 3, generator=g), torch.rand(S, generator=g) + 0.5
+    gd, gc = torch.randn(37, generator=g), torch.randn(37, 3, generator=g)
+    ours = [t.to(cuda).requires_grad_(True) for t in (a, c, d)]
+    out = st_api.compose_strokes(*ours, mode)
+    got = torch.autograd.grad(out, ours, (gd.to(cuda), gc.to(cuda)))
+    ref = [t.double().requires_grad_(True) for t in (a, c, d)]
+    key = ref[0] * ref[2] if mode == "softmax_density_weighted" else ref[0]
+    w = torch.softmax(key / 0.05, -1)
+    want = ((w * ref[0] * ref[2]).sum(-1), (w[..., None] * ref[1]).sum(-2))
+    for x, y in zip(out, want):
+        assert rel(x, y) < 1e-5
+    for x, y in zip(got, torch.autograd.grad(want, ref, (gd.double(), gc.double()))):
+        assert rel(x, y) < 1e-4
+
+
+@pytest.mark.parametrize("S,C", [(1, 3), (33, 1), (128, 3), (256, 3), (260, 1), (1000, 3)])
+@pytest.mark.parametrize("grad_mode", ["exact", "compat"])
+def test_compose_backward_write_equals_accumulation(cuda, grad_mode, S, C):
+    """The writing compose backward fills what the accumulating one adds to zeros, in the
+    vector, row and compat kernels, whatever the buffers held."""
+    from neural3dstrokes_b200 import strokelib as sl
+    g = torch.Generator().manual_seed(S)
+    a, c, d = (torch.rand(*s, generator=g).to(cuda) for s in ((53, S), (53, S, C), (S,)))
+    gd, gc = torch.randn(53, generator=g).to(cuda), torch.randn(53, C, generator=g).to(cuda)
+    before = sl.get_grad_mode()
+    sl.set_grad_mode(grad_mode)
+    try:
+        want = [torch.zeros_like(t) for t in (a, c, d)]
+        sl.compose_backward(*want, gd, gc, a, c, d)
+        got = [torch.full_like(a, float("nan")), torch.full_like(c, float("nan")), torch.zeros_like(d)]
+        sl._compose_backward("n3ds_compose_backward_write", *got, gd, gc, a, c, d)
+    finally:
+        sl.set_grad_mode(before)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert rel(got[2], want[2]) < 1e-6
