@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_con
     #pragma unroll
                 for (int j = 0; j < 16; j++) v[j] = -0.f;
                 QuadFwd qf;
-                const float sdf = quad_eval(rec, c.x, qf);
+                const float sdf = quad_eval<false>(rec, c.x, qf);
                 const float kk = h.y * c.rinv;
                 const float m = -sdf * kk;
                 const float a = mode == STEP_HARD ? (sdf <= 0.f ? 1.f : 0.f) : soft_alpha(mode, m);
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_con
     #pragma unroll
                 for (int j = 0; j < 32; j++) v[j] = -0.f;
                 CubicFwd cf;
-                const float sdf = cubic_eval(rec, c.x, cf, base == B_CATMULL_ROM);
+                const float sdf = cubic_eval<false>(rec, c.x, cf, base == B_CATMULL_ROM);
                 const float kk = h.y * c.rinv;
                 const float m = -sdf * kk;
                 const float a = mode == STEP_HARD ? (sdf <= 0.f ? 1.f : 0.f) : soft_alpha(mode, m);
@@ -920,7 +920,6 @@ __device__ void prep_stroke(const PrepLaunch& P, long long s, float* rec) {
   rec[R_COLOR + 2] = col[2];
   rec[R_DENSITY] = P.density ? P.density[s] : 0.f;
   rec[R_KFIX] = kappa / delta * (s1k ? sc.x : 1.f);
-  rec[R_DELTA] = delta;
 
   // culling: sdf_local >= Lg (|p| - rho0) with p the local point; world centre cw
   float rho0 = 1.f, Lg = 1.f, smax = fmaxf(sc.x, fmaxf(sc.y, sc.z)), smin = fminf(sc.x, fminf(sc.y, sc.z));
@@ -1028,6 +1027,10 @@ __device__ void prep_stroke(const PrepLaunch& P, long long s, float* rec) {
       curve_weights(ti, w, power);
       V3 v = P4[0] * w[0] + P4[1] * w[1] + P4[2] * w[2] + P4[3] * w[3];
       rec[R_CV + 3 * i] = v.x; rec[R_CV + 3 * i + 1] = v.y; rec[R_CV + 3 * i + 2] = v.z;
+    }
+    for (int i = 0; i < CUBIC_SEGMENTS; i++) {
+      const V3 ab = ld3(rec + R_CV + 3 * (i + 1)) - ld3(rec + R_CV + 3 * i);
+      rec[r_cinv(i)] = 1.f / dot(ab, ab);
     }
     // curve-to-polyline distance <= max|B''| dt^2 / 8, |B''| <= 6 max second difference
     // of the Bezier control points (the hull points of either curve)

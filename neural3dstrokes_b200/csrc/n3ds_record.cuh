@@ -63,11 +63,11 @@ __host__ __device__ __forceinline__ int sdf_id_param_count(int sdf_id) {
 
 // ---- record field offsets (floats). Hot fields sit in 16-byte groups so the inner
 // loops read them with 128-bit shared-memory loads (rec4(rec)[k]).
-// q0: kind word, soft-step slope, density, softness
+// q0: kind word, soft-step slope, density
 constexpr int R_KIND = 0;      // int bits
 constexpr int R_KFIX = 1;      // kappa/delta (times s for single-scale with inv_scale_radius)
 constexpr int R_DENSITY = 2;
-constexpr int R_DELTA = 3;
+// slot 3: cubic curves, see R_CINV
 // q1: colour, base parameter (round-cube radius / capsule half-length)
 constexpr int R_COLOR = 4;     // 3
 constexpr int R_BP = 7;        // first base parameter (round-cube radius, capsule / line half-length,
@@ -94,6 +94,11 @@ constexpr int R_CA = 8, R_CR1 = 11;    // q2: A, r1
 constexpr int R_CB = 12, R_CR2 = 15;   // q3: B, r2
 constexpr int R_CC = 16, R_CD = 20;    // q4, q5: C, D
 constexpr int R_CV = 24;       // 11 polyline vertices, 33 floats (24..56), read as 9 float4
+// 1 / |piece|^2 of the 10 polyline pieces, in the words the 16-byte groups leave free:
+// 3, 7, 19, 23, 57, 58, 59, 61, 62, 63
+__host__ __device__ constexpr int r_cinv(int i) {
+  return i == 0 ? 3 : i == 1 ? 7 : i == 2 ? 19 : i == 3 ? 23 : i < 7 ? 53 + i : 54 + i;
+}
 // every curve: culling radius of its polyline pieces beyond their half-length (the
 // largest tube radius plus the curve's distance bound to its polyline)
 constexpr int R_CTEST = 60;

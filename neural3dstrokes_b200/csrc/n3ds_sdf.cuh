@@ -321,11 +321,25 @@ __device__ __forceinline__ float quad_newton(float s, float pt, float q) {
   for (int it = 0; it < 2; it++) {
     const float g = (s * s + 3.f * pt) * s + q;
     const float gd = 3.f * (s * s + pt);
-    if (fabsf(gd) > 1e-12f) s -= g / gd;
+    if (fabsf(gd) > 1e-12f) s -= __fdividef(g, gd);
   }
   return s;
 }
 
+// sin and cos on [0, pi / 3] by their Taylor series (remainders below 4e-9, a sixteenth of
+// a float32 ulp of the result): no argument reduction, no slow path. For the forwards and
+// the drop-in operators; in the segment backward, whose registers are full, its constants
+// cost every primitive more than the call (16 mixed scenes 4.17 -> 4.55 ms).
+__device__ __forceinline__ void sincos_third(float v, float* s, float* c) {
+  const float v2 = v * v;
+  *s = v * fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, -1.f / 39916800.f, 1.f / 362880.f), -1.f / 5040.f), 1.f / 120.f),
+                         -1.f / 6.f),
+                1.f);
+  *c = fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, -1.f / 3628800.f, 1.f / 40320.f), -1.f / 720.f), 1.f / 24.f), -0.5f),
+            1.f);
+}
+
+template <bool TAYLOR = true>
 __device__ __forceinline__ float quad_eval(const float* rec, V3 pos, QuadFwd& s) {
   const float4 qA = rec4(rec)[R_QA / 4], qa = rec4(rec)[R_Qa / 4], qb = rec4(rec)[R_Qb / 4],
                qc = rec4(rec)[R_Qc / 4];
@@ -342,36 +356,44 @@ __device__ __forceinline__ float quad_eval(const float* rec, V3 pos, QuadFwd& s)
   const float pt = cbrtf(p3 + 2.5e-9f);
   s.pt = pt;
   float t, t_raw;
+  // The lanes of a warp take both branches, so what they share runs once after them: the
+  // refinement of the true root (s0 its start). One real root: Cardano's terms have the
+  // product -pt, so the larger one's cube root gives the other (|x| >= H / 2 >= 5e-5).
+  // Three: (m + n) z is the reference's first candidate (not a root, kept as computed),
+  // (-n - m) z a true root.
+  float s0, z = 0.f, m = 0.f, n = 0.f;
   if (h >= 0.0f) {
     s.pos_branch = 1;
-    float H = sqrtf(h + 1e-8f);
-    float x0 = (H - q) * 0.5f, x1 = -(H + q) * 0.5f;
-    float u0 = copysignf(cbrtf(fabsf(x0)), x0), u1 = copysignf(cbrtf(fabsf(x1)), x1);
-    const float sr = quad_newton(u0 + u1, pt, q);
-    s.sr = sr;
-    t_raw = sr - kx;
-    t = clampf(t_raw, 0.f, 1.f);
+    const float H = sqrtf(h + 1e-8f);
+    const float u = copysignf(cbrtf((fabsf(q) + H) * 0.5f), -q);
+    s0 = u - __fdividef(pt, u);
   } else {
     s.pos_branch = 0;
-    float z = sqrtf(-p + 1e-8f);
-    float den = p * z * 2.0f + 1e-8f;
-    float arg = q / den;
-    float v = acosf(arg) / 3.0f;
+    z = sqrtf(-p + 1e-8f);
+    s.den = p * z * 2.0f + 1e-8f;
+    s.arg = q / s.den;
+    s.v = acosf(s.arg) / 3.0f;
     float sv, cv;
-    sincosf(v, &sv, &cv);
-    float m = cv, n = sv * BEZ_SQRT3;
-    // (m + n) z is the reference's first candidate (not a root, kept as computed);
-    // (-n - m) z is a true root and is refined
-    const float sb = quad_newton((-n - m) * z, pt, q);
-    float ra = (m + n) * z - kx, rb = sb - kx;
+    if (TAYLOR) sincos_third(s.v, &sv, &cv);
+    else sincosf(s.v, &sv, &cv);
+    m = cv;
+    n = sv * BEZ_SQRT3;
+    s0 = (-n - m) * z;
+  }
+  s.sr = quad_newton(s0, pt, q);
+  const float rb = s.sr - kx;
+  if (s.pos_branch) {
+    t_raw = rb;
+    t = clampf(t_raw, 0.f, 1.f);
+  } else {
+    const float ra = (m + n) * z - kx;
     float ta = clampf(ra, 0.f, 1.f), tb = clampf(rb, 0.f, 1.f);
     V3 ea = d + (c + b * ta) * ta, eb = d + (c + b * tb) * tb;
     float da = dot(ea, ea), db = dot(eb, eb);
     bool use_b = db < da;
     t = use_b ? tb : ta;
     t_raw = use_b ? rb : ra;
-    s.sr = sb;
-    s.z = z; s.den = den; s.arg = arg; s.v = v; s.m = m; s.n = n; s.sigma = use_b ? -1.f : 1.f;
+    s.z = z; s.m = m; s.n = n; s.sigma = use_b ? -1.f : 1.f;
   }
   V3 e = d + (c + b * t) * t;
   float dist = sqrtf(dot(e, e) + 1e-8f);
@@ -507,40 +529,53 @@ struct CubicFwd {
   V3 v;     // B(t) - pos
 };
 
+template <bool INV = true>
 __device__ __forceinline__ float cubic_eval(const float* rec, V3 pos, CubicFwd& s, bool power) {
   constexpr float step = 1.0f / CUBIC_SEGMENTS;
-  float best = 1e18f, tau_best = 0.f, tau_raw_best = 0.f;
+  // Bound by issue, 10 pieces a pair: the reciprocal squared lengths come with the record
+  // (INV; else a fast division, 10 registers less, for the backward), the clamped parameter
+  // is formed again for the winner only (a NaN parameter, from a piece of length 0, clamps
+  // to 1, and a NaN distance never wins, as in the reference's loop). The distances keep
+  // the form pos - (s0 + ab t): where two pieces are nearly as close their rounding decides,
+  // and (pos - s0) - ab t, three instructions less, decided otherwise for a few samples
+  // (4e-4 of the control-point gradient's norm).
+  // 2000 mixed strokes, a quarter curves, 131,072 rays x 96, forward: 9.59 -> 8.22 ms with
+  // the quadratic's changes (quad_eval); 2000 curves, 16,411 rays x 64: forward 1.85 ->
+  // 1.65 ms, backward 1.74 -> 1.66.
+  float best = 1e18f, tau_raw_best = 0.f;
   int seg = 0;
-  float vtx[36];
+  float vtx[36], inv[CUBIC_SEGMENTS];
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     const float4 q = rec4(rec)[R_CV / 4 + k];
     vtx[4 * k] = q.x; vtx[4 * k + 1] = q.y; vtx[4 * k + 2] = q.z; vtx[4 * k + 3] = q.w;
   }
+  const float4 cA = rec4(rec)[R_CA / 4], cB = rec4(rec)[R_CB / 4], cC = rec4(rec)[R_CC / 4],
+               cD = rec4(rec)[R_CD / 4], q15 = rec4(rec)[15];
+  inv[0] = rec[r_cinv(0)]; inv[1] = rec[r_cinv(1)]; inv[2] = cC.w; inv[3] = cD.w;
+  inv[4] = vtx[33]; inv[5] = vtx[34]; inv[6] = vtx[35];
+  inv[7] = q15.y; inv[8] = q15.z; inv[9] = q15.w;
   V3 s0 = v3(vtx[0], vtx[1], vtx[2]);
 #pragma unroll
   for (int i = 1; i <= CUBIC_SEGMENTS; i++) {
     V3 s1 = v3(vtx[3 * i], vtx[3 * i + 1], vtx[3 * i + 2]);
-    V3 ab = s1 - s0;
-    float tr = dot(pos - s0, ab) / dot(ab, ab);
-    float tt = clampf(tr, 0.f, 1.f);
-    V3 dv = pos - (s0 + ab * tt);
+    V3 ab = s1 - s0, w = pos - s0;
+    float tr = INV ? dot(w, ab) * inv[i - 1] : __fdividef(dot(w, ab), dot(ab, ab));
+    V3 dv = pos - (s0 + ab * clampf(tr, 0.f, 1.f));
     float d2 = dot(dv, dv);
     if (d2 < best) {
       best = d2;
-      tau_best = tt;
       tau_raw_best = tr;
       seg = i;
     }
     s0 = s1;
   }
+  const float tau_best = seg ? clampf(tau_raw_best, 0.f, 1.f) : 0.f;
   // the winning segment's t, as the reference's t_start (1 - tau) + t_end tau with
   // t_start = (seg - 1) step, t_end = seg step (the same float values as in its loop)
   const float t_min = seg ? ((float)(seg - 1) * step) * (1.0f - tau_best) + ((float)seg * step) * tau_best : 0.f;
   float w[4];
   curve_weights(t_min, w, power);
-  const float4 cA = rec4(rec)[R_CA / 4], cB = rec4(rec)[R_CB / 4], cC = rec4(rec)[R_CC / 4],
-               cD = rec4(rec)[R_CD / 4];
   V3 P = xyz(cA) * w[0] + xyz(cB) * w[1] + xyz(cC) * w[2] + xyz(cD) * w[3];
   V3 v = P - pos;
   float dist = sqrtf(dot(v, v));
