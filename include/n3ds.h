@@ -86,6 +86,17 @@ int n3ds_stroke_backward(float* grad_shape_params, float* grad_color_params, flo
                          int inv_scale_radius, int grad_mode, void* workspace,
                          size_t workspace_bytes, n3ds_stream_t stream);
 
+/* The same, but grad_shape_params, grad_color_params and grad_x are written (they need not
+ * be cleared). */
+int n3ds_stroke_backward_write(float* grad_shape_params, float* grad_color_params, float* grad_x,
+                               const float* grad_alpha, const float* grad_color, const float* grad_sdf,
+                               const float* x, const float* radius, const float* viewdir, const float* alpha,
+                               const float* shape_params, const float* color_params, int64_t n_points,
+                               int64_t n_viewdirs, int64_t n_strokes, int64_t n_shape_params, int64_t n_color_params,
+                               uint32_t sdf_id, uint32_t color_id, float sdf_delta, int use_laplace_transform,
+                               int inv_scale_radius, int grad_mode, void* workspace, size_t workspace_bytes,
+                               n3ds_stream_t stream);
+
 /* Replaces compose_forward (compositing.cu:159-204; declared compositing.h:11-15).
  * density_out [P], color_out [P,C], alphas [P,S], colors [P,S,C], density_params [S];
  * C in {1, 3}. */

@@ -80,6 +80,9 @@ _SIGS = {
     "n3ds_stroke_backward": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, c_i64, c_i64,
                                             c_i64, c_i64, c_i64, c_u32, c_u32, ctypes.c_float, ctypes.c_int,
                                             ctypes.c_int, ctypes.c_int, _P, c_size_t, _P]),
+    "n3ds_stroke_backward_write": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, c_i64, c_i64,
+                                            c_i64, c_i64, c_i64, c_u32, c_u32, ctypes.c_float, ctypes.c_int,
+                                            ctypes.c_int, ctypes.c_int, _P, c_size_t, _P]),
     "n3ds_compose_forward": (ctypes.c_int, [_P, _P, _P, _P, _P, c_i64, c_i64, c_i64, _P]),
     "n3ds_compose_workspace_bytes": (c_size_t, [c_i64, c_i64, ctypes.c_int]),
     "n3ds_compose_backward": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_i64, c_i64, c_i64,

@@ -832,13 +832,15 @@ int n3ds_stroke_forward(float* alpha_out, float* color_out, float* sdf_out, floa
   return N3DS_OK;
 }
 
-int n3ds_stroke_backward(float* grad_shape_params, float* grad_color_params, float* grad_x, const float* grad_alpha,
-                         const float* grad_color, const float* grad_sdf, const float* x, const float* radius,
-                         const float* viewdir, const float* alpha, const float* shape_params,
-                         const float* color_params, int64_t n_points, int64_t n_viewdirs, int64_t n_strokes,
-                         int64_t n_shape_params, int64_t n_color_params, uint32_t sdf_id, uint32_t color_id,
-                         float sdf_delta, int use_laplace_transform, int inv_scale_radius, int grad_mode,
-                         void* workspace, size_t workspace_bytes, n3ds_stream_t stream) {
+// write: grad_shape_params, grad_color_params and grad_x are overwritten (the preparation
+// clears what kernels accumulate into) instead of accumulated into.
+static int stroke_backward(bool write, float* grad_shape_params, float* grad_color_params, float* grad_x,
+                           const float* grad_alpha, const float* grad_color, const float* grad_sdf, const float* x,
+                           const float* radius, const float* viewdir, const float* alpha, const float* shape_params,
+                           const float* color_params, int64_t n_points, int64_t n_viewdirs, int64_t n_strokes,
+                           int64_t n_shape_params, int64_t n_color_params, uint32_t sdf_id, uint32_t color_id,
+                           float sdf_delta, int use_laplace_transform, int inv_scale_radius, int grad_mode,
+                           void* workspace, size_t workspace_bytes, n3ds_stream_t stream) {
   int rc = check_stroke_args(sdf_id, color_id, n_points, n_viewdirs, n_strokes, n_shape_params, n_color_params, 0,
                              workspace, workspace_bytes);
   if (rc) return rc;
@@ -848,9 +850,14 @@ int n3ds_stroke_backward(float* grad_shape_params, float* grad_color_params, flo
     return fail(N3DS_ERR_INVALID, "null tensor pointer");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   StrokeWs w = stroke_ws(workspace, n_strokes);
-  n3ds::launch_prep(uniform_prep(w, shape_params, n_shape_params, color_params, n_color_params, n_strokes, sdf_id,
-                                 sdf_delta, use_laplace_transform, inv_scale_radius, true),
-                    st);
+  n3ds::PrepLaunch prep = uniform_prep(w, shape_params, n_shape_params, color_params, n_color_params, n_strokes, sdf_id,
+                                       sdf_delta, use_laplace_transform, inv_scale_radius, true);
+  if (write) {
+    prep.clear_color = grad_color_params;
+    prep.clear_x = grad_x;
+    prep.n_clear_x = grad_x ? 3 * n_points : 0;
+  }
+  n3ds::launch_prep(prep, st);
   N3DS_CUDA_TRY(cudaGetLastError());
   const int compat = grad_mode == N3DS_GRAD_COMPAT;
   if (n_points > 0) {
@@ -898,9 +905,39 @@ int n3ds_stroke_backward(float* grad_shape_params, float* grad_color_params, flo
   F.grad_density = nullptr;
   F.grad_delta = nullptr;
   F.accumulate = 1;
+  F.write_shape = write;
   n3ds::launch_finalize(F, st);
   N3DS_CUDA_TRY(cudaGetLastError());
   return N3DS_OK;
+}
+
+int n3ds_stroke_backward(float* grad_shape_params, float* grad_color_params, float* grad_x, const float* grad_alpha,
+                         const float* grad_color, const float* grad_sdf, const float* x, const float* radius,
+                         const float* viewdir, const float* alpha, const float* shape_params,
+                         const float* color_params, int64_t n_points, int64_t n_viewdirs, int64_t n_strokes,
+                         int64_t n_shape_params, int64_t n_color_params, uint32_t sdf_id, uint32_t color_id,
+                         float sdf_delta, int use_laplace_transform, int inv_scale_radius, int grad_mode,
+                         void* workspace, size_t workspace_bytes, n3ds_stream_t stream) {
+  return stroke_backward(false, grad_shape_params, grad_color_params, grad_x, grad_alpha, grad_color, grad_sdf, x,
+                         radius, viewdir, alpha, shape_params, color_params, n_points, n_viewdirs, n_strokes,
+                         n_shape_params, n_color_params, sdf_id, color_id, sdf_delta, use_laplace_transform,
+                         inv_scale_radius, grad_mode, workspace, workspace_bytes, stream);
+}
+
+int n3ds_stroke_backward_write(float* grad_shape_params, float* grad_color_params, float* grad_x,
+                               const float* grad_alpha, const float* grad_color, const float* grad_sdf, const float* x,
+                               const float* radius, const float* viewdir, const float* alpha,
+                               const float* shape_params, const float* color_params, int64_t n_points,
+                               int64_t n_viewdirs, int64_t n_strokes, int64_t n_shape_params, int64_t n_color_params,
+                               uint32_t sdf_id, uint32_t color_id, float sdf_delta, int use_laplace_transform,
+                               int inv_scale_radius, int grad_mode, void* workspace, size_t workspace_bytes,
+                               n3ds_stream_t stream) {
+  if (n_strokes == 0 && grad_x && n_points > 0)  // nothing else launches: no stroke reaches a point
+    N3DS_CUDA_TRY(cudaMemsetAsync(grad_x, 0, size_t(n_points) * 12, reinterpret_cast<cudaStream_t>(stream)));
+  return stroke_backward(true, grad_shape_params, grad_color_params, grad_x, grad_alpha, grad_color, grad_sdf, x,
+                         radius, viewdir, alpha, shape_params, color_params, n_points, n_viewdirs, n_strokes,
+                         n_shape_params, n_color_params, sdf_id, color_id, sdf_delta, use_laplace_transform,
+                         inv_scale_radius, grad_mode, workspace, workspace_bytes, stream);
 }
 
 int n3ds_compose_forward(float* density_out, float* color_out, const float* alphas, const float* colors,

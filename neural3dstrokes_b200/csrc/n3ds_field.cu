@@ -1114,6 +1114,10 @@ __global__ void __launch_bounds__(PREP_THREADS) prep_kernel(const PrepLaunch P) 
   const int n = (int)min((long long)PREP_THREADS, P.n_strokes - s0);  // <= 0: counters only
   if (P.gslots)
     for (int i = threadIdx.x; i < n * GRAD_SLOTS; i += PREP_THREADS) P.gslots[s0 * GRAD_SLOTS + i] = 0.f;
+  if (P.clear_color)
+    for (int i = threadIdx.x; i < n * P.color_stride; i += PREP_THREADS) P.clear_color[s0 * P.color_stride + i] = 0.f;
+  if (P.clear_x)
+    for (long long i = s; i < P.n_clear_x; i += (long long)gridDim.x * PREP_THREADS) P.clear_x[i] = 0.f;
   if (s < P.n_strokes) prep_stroke(P, s, rows + threadIdx.x * PITCH);
   __syncthreads();
   for (int i = threadIdx.x; i < n * REC_FLOATS; i += PREP_THREADS)
@@ -1164,7 +1168,9 @@ __global__ void finalize_kernel(const FinalizeLaunch F) {
   } else if (base <= B_TETRAHEDRON) {
     prim_param_grads(F, s, base, flags, g, rec, o);
   }
-  for (int j = 0; j < F.param_stride && j < 64; j++) put(out + j, o[j]);
+  for (int j = 0; j < F.param_stride && j < 64; j++) out[j] = acc && !F.write_shape ? out[j] + o[j] : o[j];
+  if (F.write_shape)
+    for (int j = 64; j < F.param_stride; j++) out[j] = 0.f;
 }
 
 // Primitive slots -> [base, scale (1|3), euler (3), translation (3)] gradients.
@@ -1320,6 +1326,11 @@ void launch_module_inputs(const ModuleInputs& m, cudaStream_t st) {
 
 void launch_prep(const PrepLaunch& p, cudaStream_t st) {
   long long n = p.n_strokes > p.n_counters ? p.n_strokes : p.n_counters;
+  // enough blocks to clear a large position gradient too (at most four per SM for that)
+  if (p.clear_x && n < p.n_clear_x) {
+    const long long most = 148LL * 4 * PREP_THREADS;
+    n = n > most ? n : (p.n_clear_x < most ? p.n_clear_x : most);
+  }
   if (n < 1) n = 1;
   prep_kernel<<<(unsigned)((n + PREP_THREADS - 1) / PREP_THREADS), PREP_THREADS, 0, st>>>(p);
 }

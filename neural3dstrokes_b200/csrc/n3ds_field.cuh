@@ -107,6 +107,9 @@ struct PrepLaunch {
   int* counters;
   int n_counters;
   float* gslots;           // zeroed when non-null
+  float* clear_color;      // n_strokes * color_stride floats zeroed when non-null
+  float* clear_x;          // n_clear_x floats zeroed when non-null
+  long long n_clear_x;
   unsigned long long* stats;
   int* mask_tag;           // set to mask_tag_value when non-null
   int mask_tag_value;
@@ -136,6 +139,7 @@ struct FinalizeLaunch {
   float* grad_density;     // [S]
   float* grad_delta;       // [S] or null
   int accumulate;          // 1: add into the outputs instead of overwriting
+  int write_shape;         // 1: overwrite grad_shape even so (every column, the unused ones with 0)
   int color_stride;        // floats per stroke row of grad_color (3 for the fused path)
   // optional stroke windows, as in PrepLaunch: strokes outside [frozen, active) get
   // zero gradients

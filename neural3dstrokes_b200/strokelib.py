@@ -71,7 +71,7 @@ def stroke_forward(alpha_output, color_output, sdf_output, texcoord_output, x, r
           "alpha_output / color_output are too small")
     _need(sdf_output.numel() == 0 or sdf_output.numel() >= P * S, "sdf_output is too small")
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _lib.device_guard(x.device):
         ws_bytes = lib.n3ds_stroke_workspace_bytes(S)
         ws = _lib.workspace(ws_bytes, x.device)
         rc = lib.n3ds_stroke_forward(
@@ -89,6 +89,16 @@ def stroke_backward(grad_shape_params, grad_color_params, grad_x, grad_alpha, gr
                     radius, viewdir, alpha, shape_params, color_params, sdf_id, color_id, sdf_delta,
                     use_laplace_transform, inv_scale_radius):
     """strokes_backward.cu:224-287: accumulates grad_shape_params, grad_color_params, grad_x."""
+    _stroke_backward("n3ds_stroke_backward", grad_shape_params, grad_color_params, grad_x, grad_alpha, grad_color,
+                     grad_sdf, x, radius, viewdir, alpha, shape_params, color_params, sdf_id, color_id, sdf_delta,
+                     use_laplace_transform, inv_scale_radius)
+
+
+def _stroke_backward(entry, grad_shape_params, grad_color_params, grad_x, grad_alpha, grad_color, grad_sdf, x,
+                     radius, viewdir, alpha, shape_params, color_params, sdf_id, color_id, sdf_delta,
+                     use_laplace_transform, inv_scale_radius):
+    """``entry``: n3ds_stroke_backward, or n3ds_stroke_backward_write, which stores the
+    gradients instead of adding to them."""
     names = ["grad_shape_params", "grad_color_params", "grad_x", "grad_alpha", "grad_color", "grad_sdf",
              "x", "radius", "viewdir", "shape_params", "color_params"]
     ts = [grad_shape_params, grad_color_params, grad_x, grad_alpha, grad_color, grad_sdf, x, radius, viewdir,
@@ -103,10 +113,10 @@ def stroke_backward(grad_shape_params, grad_color_params, grad_x, grad_alpha, gr
     _need(grad_shape_params.shape == shape_params.shape and grad_color_params.shape == color_params.shape,
           "gradient buffers must match the parameter shapes")
     lib = _lib.load()
-    with torch.cuda.device(x.device):
+    with _lib.device_guard(x.device):
         ws_bytes = lib.n3ds_stroke_workspace_bytes(S)
         ws = _lib.workspace(ws_bytes, x.device)
-        rc = lib.n3ds_stroke_backward(
+        rc = getattr(lib, entry)(
             _lib.ptr(grad_shape_params), _lib.ptr(grad_color_params), _lib.ptr(grad_x), _lib.ptr(grad_alpha),
             _lib.ptr(grad_color), _lib.ptr(grad_sdf), _lib.ptr(x), _lib.ptr(radius), _lib.ptr(viewdir),
             _lib.ptr(alpha), _lib.ptr(shape_params), _lib.ptr(color_params), P, viewdir.size(0), S,
@@ -126,7 +136,7 @@ def compose_forward(density_output, color_output, alphas, colors, density_params
     _need(colors.numel() == P * S * C and density_params.numel() >= S, "colors / density_params shape mismatch")
     _need(density_output.numel() >= P and color_output.numel() >= P * C, "outputs are too small")
     lib = _lib.load()
-    with torch.cuda.device(alphas.device):
+    with _lib.device_guard(alphas.device):
         rc = lib.n3ds_compose_forward(_lib.ptr(density_output), _lib.ptr(color_output), _lib.ptr(alphas),
                                       _lib.ptr(colors), _lib.ptr(density_params), P, S, C, _lib.stream_ptr())
     _lib.check(rc)
@@ -155,7 +165,7 @@ def _compose_backward(entry, grad_alphas, grad_colors, grad_density_params, grad
     _need(grad_density_output.numel() in (0, P) and grad_color_output.numel() in (0, P * C),
           "upstream gradient shape mismatch")
     lib = _lib.load()
-    with torch.cuda.device(alphas.device):
+    with _lib.device_guard(alphas.device):
         ws_bytes = lib.n3ds_compose_workspace_bytes(P, S, _grad_mode)
         ws = _lib.workspace(ws_bytes, alphas.device) if ws_bytes else None
         rc = getattr(lib, entry)(

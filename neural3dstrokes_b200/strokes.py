@@ -129,11 +129,10 @@ class _StrokeFn(torch.autograd.Function):
         g_color = (torch.zeros(x.shape[0], S, _COLOR_DIM, device=dev) if g_color is None
                    else g_color.contiguous().float().reshape(-1, S, _COLOR_DIM))
         g_sdf = torch.empty(0, device=dev) if g_sdf is None else g_sdf.contiguous().float().reshape(-1, S)
-        gs = torch.zeros_like(shape_params)
-        gc = torch.zeros_like(color_params)
-        gx = torch.zeros_like(x) if ctx.needs_input_grad[0] else torch.empty(0, device=dev)
-        _backend.stroke_backward(gs, gc, gx, g_alpha, g_color, g_sdf, x, radius, viewdir, alpha, shape_params,
-                                 color_params, sdf_id, color_id, sdf_delta, lap, inv)
+        gs, gc = torch.empty_like(shape_params), torch.empty_like(color_params)
+        gx = torch.empty_like(x) if ctx.needs_input_grad[0] else torch.empty(0, device=dev)
+        _backend._stroke_backward("n3ds_stroke_backward_write", gs, gc, gx, g_alpha, g_color, g_sdf, x, radius, viewdir,
+                                  alpha, shape_params, color_params, sdf_id, color_id, sdf_delta, lap, inv)
         gx = gx.reshape(*pre, 3) if ctx.needs_input_grad[0] else None
         return gx, None, None, gs, gc, None, None, None, None, None, None, None
 
