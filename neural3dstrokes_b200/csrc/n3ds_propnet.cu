@@ -771,11 +771,19 @@ __global__ void __launch_bounds__(kTile, SCATTER ? 3 : FP_CTAS(C * LMAX)) densit
         else if (i == (int)P.F) atomicAdd(P.g_b1 + j, w2j * v[i]);
       }
     }
+    // dW2 and db2: the warps' sums first, one atomic per value and CTA (a quarter of the
+    // order-dependent rounding; the tensor cores are done with the feature tile)
+    float* part = reinterpret_cast<float*>(smem + SL.bp);
     if ((lane & 1) == 0) {
 #pragma unroll
-      for (int c = 0; c < kHidden / 16; c++) atomicAdd(P.g_w2 + c * 16 + (lane >> 1), acc_w2[c]);
+      for (int c = 0; c < kHidden / 16; c++) part[warp * (kHidden + 1) + c * 16 + (lane >> 1)] = acc_w2[c];
     }
-    if (lane == 0) atomicAdd(P.g_b2, acc_b2);
+    if (lane == 0) part[warp * (kHidden + 1) + kHidden] = acc_b2;
+    __syncthreads();
+    if (tid <= kHidden) {
+      const float s = (part[tid] + part[(kHidden + 1) + tid]) + (part[2 * (kHidden + 1) + tid] + part[3 * (kHidden + 1) + tid]);
+      atomicAdd(tid < kHidden ? P.g_w2 + tid : P.g_b2, s);
+    }
   }
   teardown(P, M, phase, timed_out, kColsBwd);
 }
