@@ -398,6 +398,16 @@ int n3ds_resample_intervals(float* s_out, float* t_out, const float* sdist, cons
                             const float* jitter, int32_t single_jitter, float domain_lo, float domain_hi,
                             const float* near, const float* far, n3ds_stream_t stream);
 
+/* A proposal level's samples (cast_rays, render.py:5-26): coords [R, N, 3] = directions * t +
+ * origins and radius [R, N] = radii * t at the midpoints t of tdist [R, N + 1]. */
+int n3ds_ray_points(float* coords, float* radius, const float* tdist, const float* origins, const float* directions,
+                    const float* radii, int64_t n_rays, int32_t n_samples, n3ds_stream_t stream);
+
+/* The weights of compute_alpha_weights (render.py:29-48): [R, N] from density [R, N], tdist
+ * [R, N + 1] and directions [R, 3]. */
+int n3ds_ray_weights(float* weights, const float* density, const float* tdist, const float* directions, int64_t n_rays,
+                     int32_t n_samples, int32_t opaque_background, n3ds_stream_t stream);
+
 /* Stroke insertion and reset on the device: StrokeField.step_update
  * (source/models.py:586-658) with the stroke count in device memory, so a training
  * step needs no host round trip. */

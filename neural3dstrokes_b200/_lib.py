@@ -110,6 +110,8 @@ _SIGS = {
     "n3ds_resample_intervals": (ctypes.c_int, [_P, _P, _P, _P, c_i64, c_i32, c_i32, ctypes.c_float,
                                                ctypes.c_float, _P, c_i32, ctypes.c_float, ctypes.c_float, _P, _P,
                                                _P]),
+    "n3ds_ray_points": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, c_i64, c_i32, _P]),
+    "n3ds_ray_weights": (ctypes.c_int, [_P, _P, _P, _P, c_i64, c_i32, c_i32, _P]),
     "n3ds_insert_workspace_bytes": (c_size_t, [_P, _P]),
     "n3ds_insert_step": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_i64, c_i32, ctypes.c_float, _P, _P, c_i64,
                                         _P, c_size_t, _P]),

@@ -9,8 +9,8 @@ Per proposal level:
     coord.py:56-99 with raydist_fn None, the Model default);
   * cast_rays (render.py:5-26) and the proposal network (mlp.PropMLP: coordinate warp,
     hash-grid encoding and density layers in one launch);
-  * compute_alpha_weights (render.py:29-48: elementwise ops and a cumulative sum over
-    [R, N], torch ops as in the reference).
+  * compute_alpha_weights (render.py:29-48): one launch without gradient, else torch ops
+    as in the reference. The samples are cast in one launch too.
 The last level's intervals are resampled the same way and returned: the stroke field
 casts its samples from them inside its kernels (field.render_rays), so the last
 level's [R, N, 3] positions are never written to memory.
@@ -25,7 +25,7 @@ from typing import List, Sequence
 
 import torch
 
-from . import stepfun
+from . import _lib, stepfun
 
 
 def compute_alpha_weights(density: torch.Tensor, tdist: torch.Tensor, dirs: torch.Tensor,
@@ -40,6 +40,42 @@ def compute_alpha_weights(density: torch.Tensor, tdist: torch.Tensor, dirs: torc
     trans = torch.exp(-torch.cat([torch.zeros_like(density_delta[..., :1]),
                                   torch.cumsum(density_delta[..., :-1], dim=-1)], dim=-1))
     return alpha * trans, alpha, trans
+
+
+def _plain(*ts):
+    """Float32 tensors on one CUDA device that no autograd graph goes back through."""
+    return all(t.is_cuda and t.dtype == torch.float32 and t.device == ts[0].device for t in ts) and \
+        not (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
+
+
+def _cast(tdist, origins, directions, radii):
+    """Sample positions [R * n, 3] and radii [R * n] at the interval midpoints."""
+    R, n = tdist.shape[0], tdist.shape[1] - 1
+    if not _plain(tdist, origins, directions, radii):
+        t = (tdist[:, :-1] + tdist[:, 1:]) / 2
+        coords = directions[:, None, :] * t[..., None] + origins[:, None, :]
+        return coords.reshape(-1, 3), (radii.reshape(R, 1) * t).reshape(-1)
+    coords = torch.empty(R * n, 3, device=tdist.device)
+    radius = torch.empty(R * n, device=tdist.device)
+    with _lib.device_guard(tdist.device):
+        t, o, d, r = (v.contiguous() for v in (tdist, origins, directions, radii))
+        _lib.check(_lib.load().n3ds_ray_points(_lib.ptr(coords), _lib.ptr(radius), _lib.ptr(t), _lib.ptr(o),
+                                               _lib.ptr(d), _lib.ptr(r), R, n, _lib.stream_ptr(tdist.device)))
+    return coords, radius
+
+
+def _weights(density, tdist, directions, opaque_background):
+    """The weights of compute_alpha_weights: one launch where they are data (no gradient),
+    else the differentiable torch operations."""
+    if not _plain(density, tdist, directions):
+        return compute_alpha_weights(density, tdist, directions, opaque_background)[0]
+    R, n = density.shape
+    out = torch.empty(R, n, device=density.device)
+    with _lib.device_guard(density.device):
+        s, t, d = density.contiguous(), tdist.contiguous(), directions.contiguous()
+        _lib.check(_lib.load().n3ds_ray_weights(_lib.ptr(out), _lib.ptr(s), _lib.ptr(t), _lib.ptr(d), R, n,
+                                                int(bool(opaque_background)), _lib.stream_ptr(density.device)))
+    return out
 
 
 @dataclasses.dataclass
@@ -90,10 +126,8 @@ def sample_rays(origins: torch.Tensor, directions: torch.Tensor, radii: torch.Te
                                                   domain=(init_s_near, init_s_far), near=near, far=far)
         if not is_prop:
             return RaySamples(sdist, tdist, levels)
-        t = (tdist[:, :-1] + tdist[:, 1:]) / 2
-        coords = directions[:, None, :] * t[..., None] + origins[:, None, :]
-        radius = radii.reshape(R, 1) * t
-        density = prop_mlps[i](coords.reshape(-1, 3), radius.reshape(-1))["density"].reshape(R, n)
-        weights = compute_alpha_weights(density, tdist, directions, opaque_background)[0]
+        coords, radius = _cast(tdist, origins, directions, radii)
+        density = prop_mlps[i](coords, radius)["density"].reshape(R, n)
+        weights = _weights(density, tdist, directions, opaque_background)
         levels.append(dict(sdist=sdist, tdist=tdist, density=density, weights=weights))
     raise AssertionError("unreachable")

@@ -162,3 +162,26 @@ def test_without_proposal_samples_the_last_level_samples_the_whole_ray(cuda):
     ref_s, _ = ost.resample_level(torch.tensor([[0.0, 1.0]]).expand(R, 2), torch.ones(R, 1), N_NERF, None, True,
                                   DIL_BIAS + DIL_MULT, 0.0, (0.0, 1.0), near.cpu()[:, None], far.cpu()[:, None])
     assert torch.allclose(out.sdist.cpu(), ref_s, atol=1e-6)
+
+
+@pytest.mark.parametrize("R,n", [(1, 2), (7, 31), (8, 32), (9, 33), (100, 64), (257, 65)])
+@pytest.mark.parametrize("opaque", [False, True])
+def test_level_kernels_match_tensor_operations(cuda, R, n, opaque):
+    """The one-launch sample cast equals the torch operations bit for bit (strided inputs
+    too), the one-launch weights float64 to 1e-6 of the largest; inputs that need a gradient
+    keep the differentiable operations."""
+    g = torch.Generator(device=cuda).manual_seed(R)
+    o, d, radii, _, _ = rays(cuda, R)
+    post = torch.sort(torch.rand(R, n + 1, generator=g, device=cuda), -1).values * 3
+    wide = torch.stack([post, post], -1)[..., 0]  # the same values, strided
+    dens = torch.rand(R, n, generator=g, device=cuda) * 5
+    t = (post[:, :-1] + post[:, 1:]) / 2
+    want = d[:, None, :] * t[..., None] + o[:, None, :]
+    for td in (post, wide):
+        coords, radius = sampler._cast(td, o, d, radii.reshape(R, 1))
+        assert torch.equal(coords, want.reshape(-1, 3)) and torch.equal(radius, (radii[:, None] * t).reshape(-1))
+        w = sampler._weights(dens, td, d, opaque)
+        ref = sampler.compute_alpha_weights(dens.double(), post.double(), d.double(), opaque)[0]
+        assert float((w - ref).abs().max()) < 1e-6
+    leaf = dens.clone().requires_grad_(True)
+    assert sampler._weights(leaf, post, d, opaque).requires_grad
