@@ -574,13 +574,13 @@ __global__ void __launch_bounds__(WARPS * 32, 1) run_bwd_kernel(const __grid_con
               g = prim_backprop(rec, kind, pl, -kk * dm, K, v, compat);
             } else if (bse == B_QUAD_BEZIER) {
               QuadFwd qf;
-              const float sdf = quad_eval(rec, x, qf);
+              const float sdf = quad_eval<false>(rec, x, qf);
               const float kk = h.y * rinv;
               v[G_K] = -sdf * kk * dm;
               g = quad_adjoint(rec, qf, -kk * dm, v + G_CTRL);
             } else {
               CubicFwd cf;
-              const float sdf = cubic_eval(rec, x, cf, bse == B_CATMULL_ROM);
+              const float sdf = cubic_eval<false>(rec, x, cf, bse == B_CATMULL_ROM);
               const float kk = h.y * rinv;
               const float dsdf = -kk * dm;
               v[G_K] = -sdf * kk * dm;

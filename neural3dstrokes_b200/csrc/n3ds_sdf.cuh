@@ -327,9 +327,9 @@ __device__ __forceinline__ float quad_newton(float s, float pt, float q) {
 }
 
 // sin and cos on [0, pi / 3] by their Taylor series (remainders below 4e-9, a sixteenth of
-// a float32 ulp of the result): no argument reduction, no slow path. For the forwards and
-// the drop-in operators; in the segment backward, whose registers are full, its constants
-// cost every primitive more than the call (16 mixed scenes 4.17 -> 4.55 ms).
+// a float32 ulp of the result): no argument reduction, no slow path. For the forwards;
+// in the segment backward, whose registers are full, its constants cost every primitive
+// more than the call (16 mixed scenes 4.17 -> 4.55 ms).
 __device__ __forceinline__ void sincos_third(float v, float* s, float* c) {
   const float v2 = v * v;
   *s = v * fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, -1.f / 39916800.f, 1.f / 362880.f), -1.f / 5040.f), 1.f / 120.f),
@@ -339,7 +339,11 @@ __device__ __forceinline__ void sincos_third(float v, float* s, float* c) {
             1.f);
 }
 
-template <bool TAYLOR = true>
+// FAST (forwards): the second Cardano term from the first, and the trigonometric root by
+// sincos_third. The backwards keep the two cube roots and sincosf: the parameter's clamp to
+// [0, 1] switches its gradient, and a start that differs in the last place moves a few
+// samples across it (1e-4 of the control-point gradient's norm).
+template <bool FAST = true>
 __device__ __forceinline__ float quad_eval(const float* rec, V3 pos, QuadFwd& s) {
   const float4 qA = rec4(rec)[R_QA / 4], qa = rec4(rec)[R_Qa / 4], qb = rec4(rec)[R_Qb / 4],
                qc = rec4(rec)[R_Qc / 4];
@@ -365,8 +369,13 @@ __device__ __forceinline__ float quad_eval(const float* rec, V3 pos, QuadFwd& s)
   if (h >= 0.0f) {
     s.pos_branch = 1;
     const float H = sqrtf(h + 1e-8f);
-    const float u = copysignf(cbrtf((fabsf(q) + H) * 0.5f), -q);
-    s0 = u - __fdividef(pt, u);
+    if (FAST) {
+      const float u = copysignf(cbrtf((fabsf(q) + H) * 0.5f), -q);
+      s0 = u - __fdividef(pt, u);
+    } else {
+      const float x0 = (H - q) * 0.5f, x1 = -(H + q) * 0.5f;
+      s0 = copysignf(cbrtf(fabsf(x0)), x0) + copysignf(cbrtf(fabsf(x1)), x1);
+    }
   } else {
     s.pos_branch = 0;
     z = sqrtf(-p + 1e-8f);
@@ -374,7 +383,7 @@ __device__ __forceinline__ float quad_eval(const float* rec, V3 pos, QuadFwd& s)
     s.arg = q / s.den;
     s.v = acosf(s.arg) / 3.0f;
     float sv, cv;
-    if (TAYLOR) sincos_third(s.v, &sv, &cv);
+    if (FAST) sincos_third(s.v, &sv, &cv);
     else sincosf(s.v, &sv, &cv);
     m = cv;
     n = sv * BEZ_SQRT3;
@@ -529,6 +538,8 @@ struct CubicFwd {
   V3 v;     // B(t) - pos
 };
 
+// INV (forwards): divisions by the segment's length squared as products with the record's
+// reciprocal. The backwards divide, for the same reason as quad_eval's.
 template <bool INV = true>
 __device__ __forceinline__ float cubic_eval(const float* rec, V3 pos, CubicFwd& s, bool power) {
   constexpr float step = 1.0f / CUBIC_SEGMENTS;
