@@ -385,10 +385,12 @@ def test_odd_level_offsets(cuda, C, dtype):
 @pytest.mark.parametrize("dtype,C", [(torch.float16, 1), (torch.float32, 1), (torch.float16, 4), (torch.float32, 4),
                                      (torch.float32, 8), (torch.float64, 8)])
 @pytest.mark.parametrize("B,L", [(1, 2), (63, 10), (64, 16), (65, 3), (1000, 10), (130, 400)])
-def test_level_rows_transposition_is_exact(cuda, B, L, C, dtype):
+def test_level_rows_transposition_is_exact(cuda, monkeypatch, B, L, C, dtype):
     """[L, B, C] <-> [B, L * C] through the tiled kernel at tile edges (and rows too long
     for it, which take the strided copy) equals torch's permutation bit for bit."""
     from neural3dstrokes_b200 import gridencoder as ge
+    monkeypatch.setattr(ge, "_TRANSPOSE_BYTES", 0)
+    monkeypatch.setattr(ge, "_TRANSPOSE_UNIT", 1)
     t = torch.randn(L, B, C, device=cuda).to(dtype)
     rows = ge._rows_of_levels(t, B, L, C)
     assert rows.is_contiguous() and torch.equal(rows, t.permute(1, 0, 2).reshape(B, L * C))
