@@ -24,6 +24,7 @@ import dataclasses
 from typing import List, Sequence
 
 import torch
+import torch.autograd.forward_ad as forward_ad
 
 from . import _lib, stepfun
 
@@ -43,9 +44,11 @@ def compute_alpha_weights(density: torch.Tensor, tdist: torch.Tensor, dirs: torc
 
 
 def _plain(*ts):
-    """Float32 tensors on one CUDA device that no autograd graph goes back through."""
+    """Float32 tensors on one CUDA device that no derivative is taken through: neither an
+    autograd graph goes back through them nor does one carry a forward-mode tangent."""
     return all(t.is_cuda and t.dtype == torch.float32 and t.device == ts[0].device for t in ts) and \
-        not (torch.is_grad_enabled() and any(t.requires_grad for t in ts))
+        not (torch.is_grad_enabled() and any(t.requires_grad for t in ts)) and \
+        all(forward_ad.unpack_dual(t).tangent is None for t in ts)
 
 
 def _cast(tdist, origins, directions, radii):

@@ -185,3 +185,53 @@ def test_level_kernels_match_tensor_operations(cuda, R, n, opaque):
         assert float((w - ref).abs().max()) < 1e-6
     leaf = dens.clone().requires_grad_(True)
     assert sampler._weights(leaf, post, d, opaque).requires_grad
+
+
+def _torch_density(gain, coords):
+    return F.softplus(4.0 * (coords * gain).sum(-1))
+
+
+class _TorchProposal(torch.nn.Module):
+    """A proposal network of plain torch operations (sample_rays takes any module)."""
+
+    def __init__(self, gain):
+        super().__init__()
+        self.gain = gain
+
+    def forward(self, coords, radius):
+        return dict(density=_torch_density(self.gain, coords))
+
+
+@pytest.mark.parametrize("opaque", [False, True])
+def test_forward_mode_tangents_pass_through_the_levels(cuda, opaque):
+    """Forward-mode derivatives (torch.autograd.forward_ad) of a torch proposal network's
+    parameters and of the rays reach the level's density and weights, against the float64
+    derivative at the same posts; the package's own networks refuse a dual ray."""
+    import torch.autograd.forward_ad as fwad
+    o, d, radii, near, far = rays(cuda, 65)
+    g = torch.Generator().manual_seed(8)
+    gain, t_gain = torch.randn(3, generator=g).to(cuda), torch.randn(3, generator=g).to(cuda)
+    t_o = torch.randn(65, 3, generator=g).to(cuda)
+    for moved in ("gain", "origins"):
+        with fwad.dual_level():
+            gain_d = fwad.make_dual(gain, t_gain) if moved == "gain" else gain
+            o_d = fwad.make_dual(o, t_o) if moved == "origins" else o
+            lv = sampler.sample_rays(o_d, d, radii, near, far, [_TorchProposal(gain_d)], 33, 8,
+                                     opaque_background=opaque).levels[0]
+            got = [fwad.unpack_dual(lv[k]) for k in ("density", "weights")]
+            got = [(v.primal.clone(), None if v.tangent is None else v.tangent.clone()) for v in got]
+        td, d64 = lv["tdist"].double(), d.double()
+
+        def chain(gain64, o64):
+            t = (td[:, :-1] + td[:, 1:]) / 2
+            dens = _torch_density(gain64, d64[:, None] * t[..., None] + o64[:, None])
+            return dens, sampler.compute_alpha_weights(dens, td, d64, opaque)[0]
+
+        z = torch.zeros_like
+        tangents = (t_gain.double(), z(o).double()) if moved == "gain" else (z(gain).double(), t_o.double())
+        want, t_want = torch.func.jvp(chain, (gain.double(), o.double()), tangents)
+        for (p, t), pw, tw in zip(got, want, t_want):
+            assert t is not None, moved
+            assert rel(p, pw) < FWD_TOL and rel(t, tw) < 1e-4
+    with fwad.dual_level(), pytest.raises(NotImplementedError):
+        sampler.sample_rays(fwad.make_dual(o, t_o), d, radii, near, far, prop_nets(cuda)[:1], 33, 8)
