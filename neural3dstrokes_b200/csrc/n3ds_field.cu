@@ -409,9 +409,11 @@ struct CompAdj {
 };
 
 // Compose step + exact adjoint for one stroke; returns dL/dm. Writes colour /
-// density slots. The prefixes repeat the forward's accumulations bit for bit, so a
-// suffix (total minus prefix) carries rounding of the strokes below alone and is exactly
-// zero behind an opaque stroke. (One running scalar for the upstream-weighted suffix
+// density slots. The prefixes repeat the forward's accumulations bit for bit (the curves'
+// evaluation spells out its fused products for that), so a suffix (total minus prefix)
+// carries rounding of the strokes below alone and is exactly zero behind an opaque stroke,
+// but for alphas below the skip threshold, which the block masks may leave out of the
+// prefixes. (One running scalar for the upstream-weighted suffix
 // takes 9 floats less, so 32 warps fit, 3.93 ms; but its rounding against the forward's
 // totals raised the softness gradient's error from 1.5e-6 to 2.2e-6 of its norm.)
 // compat: the reference compose adjoint (compositing.cu:104-155).
@@ -617,7 +619,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_con
     #pragma unroll
                 for (int j = 0; j < 16; j++) v[j] = -0.f;
                 QuadFwd qf;
-                const float sdf = quad_eval<false>(rec, c.x, qf);
+                const float sdf = quad_eval(rec, c.x, qf);
                 const float kk = h.y * c.rinv;
                 const float m = -sdf * kk;
                 const float a = mode == STEP_HARD ? (sdf <= 0.f ? 1.f : 0.f) : soft_alpha(mode, m);
@@ -1030,7 +1032,7 @@ __device__ void prep_stroke(const PrepLaunch& P, long long s, float* rec) {
     }
     for (int i = 0; i < CUBIC_SEGMENTS; i++) {
       const V3 ab = ld3(rec + R_CV + 3 * (i + 1)) - ld3(rec + R_CV + 3 * i);
-      rec[r_cinv(i)] = 1.f / dot(ab, ab);
+      rec[r_cinv(i)] = 1.f / dot_fma(ab, ab);
     }
     // curve-to-polyline distance <= max|B''| dt^2 / 8, |B''| <= 6 max second difference
     // of the Bezier control points (the hull points of either curve)

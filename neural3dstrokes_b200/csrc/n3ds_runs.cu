@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) run_bwd_kernel(const __grid_con
               g = prim_backprop(rec, kind, pl, -kk * dm, K, v, compat);
             } else if (bse == B_QUAD_BEZIER) {
               QuadFwd qf;
-              const float sdf = quad_eval<false>(rec, x, qf);
+              const float sdf = quad_eval(rec, x, qf);
               const float kk = h.y * rinv;
               v[G_K] = -sdf * kk * dm;
               g = quad_adjoint(rec, qf, -kk * dm, v + G_CTRL);

@@ -308,7 +308,7 @@ struct QuadFwd {
   float kx, ky, p, q;
   float sr, pt;  // refined depressed-cubic root s = t_raw + kx and the regularised p
   // h < 0 branch
-  float z, den, arg, v, m, n, sigma;  // sigma = +1 for the (m+n) candidate, -1 for -(m+n)
+  float z, den, arg, v, mn, sigma;  // mn = m + n; sigma = +1 for the (m+n) candidate, -1 for -(m+n)
   int pos_branch;
 };
 
@@ -319,96 +319,89 @@ struct QuadFwd {
 __device__ __forceinline__ float quad_newton(float s, float pt, float q) {
 #pragma unroll
   for (int it = 0; it < 2; it++) {
-    const float g = (s * s + 3.f * pt) * s + q;
-    const float gd = 3.f * (s * s + pt);
-    if (fabsf(gd) > 1e-12f) s -= __fdividef(g, gd);
+    const float g = fmaf(fmaf(s, s, __fmul_rn(3.f, pt)), s, q);
+    const float gd = __fmul_rn(3.f, fmaf(s, s, pt));
+    if (fabsf(gd) > 1e-12f) s = __fsub_rn(s, __fdividef(g, gd));
   }
   return s;
 }
 
 // sin and cos on [0, pi / 3] by their Taylor series (remainders below 4e-9, a sixteenth of
-// a float32 ulp of the result): no argument reduction, no slow path. For the forwards;
-// in the segment backward, whose registers are full, its constants cost every primitive
-// more than the call (16 mixed scenes 4.17 -> 4.55 ms).
+// a float32 ulp of the result): no argument reduction, no slow path.
 __device__ __forceinline__ void sincos_third(float v, float* s, float* c) {
-  const float v2 = v * v;
-  *s = v * fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, -1.f / 39916800.f, 1.f / 362880.f), -1.f / 5040.f), 1.f / 120.f),
-                         -1.f / 6.f),
-                1.f);
+  const float v2 = __fmul_rn(v, v);
+  *s = __fmul_rn(v, fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, -1.f / 39916800.f, 1.f / 362880.f), -1.f / 5040.f),
+                                           1.f / 120.f),
+                                  -1.f / 6.f),
+                         1.f));
   *c = fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, fmaf(v2, -1.f / 3628800.f, 1.f / 40320.f), -1.f / 720.f), 1.f / 24.f), -0.5f),
             1.f);
 }
 
-// FAST (forwards): the second Cardano term from the first, and the trigonometric root by
-// sincos_third. The backwards keep the two cube roots and sincosf: the parameter's clamp to
-// [0, 1] switches its gradient, and a start that differs in the last place moves a few
-// samples across it (1e-4 of the control-point gradient's norm).
-template <bool FAST = true>
+// One form for forwards and backwards, with every product that an addition could absorb
+// written as fmaf or as a rounded product: a backward then repeats its forward's value bit
+// for bit, whatever else its kernel keeps of the evaluation. (With plain expressions each
+// kernel's compilation chose the fused products itself, and the two differed in the last
+// place; so did two cube roots and sincosf in the backwards alone. At 28 warps the series
+// costs the segment backward nothing: 16 mixed scenes 4.17 -> 4.17 ms.)
+// Cardano's terms have the product -pt, so the larger one's cube root gives the other.
 __device__ __forceinline__ float quad_eval(const float* rec, V3 pos, QuadFwd& s) {
   const float4 qA = rec4(rec)[R_QA / 4], qa = rec4(rec)[R_Qa / 4], qb = rec4(rec)[R_Qb / 4],
                qc = rec4(rec)[R_Qc / 4];
   V3 A = xyz(qA), a = xyz(qa), b = xyz(qb), c = xyz(qc);
   float kk = qA.w, kx = qa.w;
   V3 d = A - pos;
-  float ky = kk * (qb.w + dot(d, b)) / 3.0f;
-  float kz = kk * dot(d, a);
-  float p = ky - kx * kx;
-  float p3 = p * p * p;
-  float q = kx * (2.0f * kx * kx - 3.0f * ky) + kz;
-  float h = q * q + 4.0f * p3;
+  float ky = __fmul_rn(kk, __fadd_rn(qb.w, dot_fma(d, b))) / 3.0f;
+  float p = fmaf(-kx, kx, ky);
+  const float pp = __fmul_rn(p, p);
+  float q = fmaf(kk, dot_fma(d, a), __fmul_rn(kx, fmaf(2.0f * kx, kx, -__fmul_rn(3.0f, ky))));
+  float h = fmaf(q, q, 4.0f * __fmul_rn(pp, p));
   s.d = d; s.kx = kx; s.ky = ky; s.p = p; s.q = q;
-  const float pt = cbrtf(p3 + 2.5e-9f);
+  const float pt = cbrtf(fmaf(pp, p, 2.5e-9f));
   s.pt = pt;
   float t, t_raw;
   // The lanes of a warp take both branches, so what they share runs once after them: the
-  // refinement of the true root (s0 its start). One real root: Cardano's terms have the
-  // product -pt, so the larger one's cube root gives the other (|x| >= H / 2 >= 5e-5).
-  // Three: (m + n) z is the reference's first candidate (not a root, kept as computed),
-  // (-n - m) z a true root.
-  float s0, z = 0.f, m = 0.f, n = 0.f;
+  // refinement of the true root (s0 its start). One real root: Cardano's two terms (the
+  // larger is at least H / 2 >= 5e-5). Three: (m + n) z is the reference's first candidate
+  // (not a root, kept as computed), (-n - m) z a true root.
+  float s0, z = 0.f, mn = 0.f;
   if (h >= 0.0f) {
     s.pos_branch = 1;
-    const float H = sqrtf(h + 1e-8f);
-    if (FAST) {
-      const float u = copysignf(cbrtf((fabsf(q) + H) * 0.5f), -q);
-      s0 = u - __fdividef(pt, u);
-    } else {
-      const float x0 = (H - q) * 0.5f, x1 = -(H + q) * 0.5f;
-      s0 = copysignf(cbrtf(fabsf(x0)), x0) + copysignf(cbrtf(fabsf(x1)), x1);
-    }
+    const float H = sqrtf(__fadd_rn(h, 1e-8f));
+    const float u = copysignf(cbrtf(__fadd_rn(fabsf(q), H) * 0.5f), -q);
+    s0 = __fsub_rn(u, __fdividef(pt, u));
   } else {
     s.pos_branch = 0;
-    z = sqrtf(-p + 1e-8f);
-    s.den = p * z * 2.0f + 1e-8f;
+    z = sqrtf(__fadd_rn(-p, 1e-8f));
+    s.den = fmaf(__fmul_rn(p, z), 2.0f, 1e-8f);
     s.arg = q / s.den;
     s.v = acosf(s.arg) / 3.0f;
     float sv, cv;
-    if (FAST) sincos_third(s.v, &sv, &cv);
-    else sincosf(s.v, &sv, &cv);
-    m = cv;
-    n = sv * BEZ_SQRT3;
-    s0 = (-n - m) * z;
+    sincos_third(s.v, &sv, &cv);
+    mn = __fadd_rn(cv, __fmul_rn(sv, BEZ_SQRT3));
+    s.z = z; s.mn = mn;
+    s0 = __fmul_rn(-mn, z);
   }
   s.sr = quad_newton(s0, pt, q);
-  const float rb = s.sr - kx;
+  const float rb = __fsub_rn(s.sr, kx);
   if (s.pos_branch) {
     t_raw = rb;
     t = clampf(t_raw, 0.f, 1.f);
   } else {
-    const float ra = (m + n) * z - kx;
+    const float ra = fmaf(mn, z, -kx);
     float ta = clampf(ra, 0.f, 1.f), tb = clampf(rb, 0.f, 1.f);
-    V3 ea = d + (c + b * ta) * ta, eb = d + (c + b * tb) * tb;
-    float da = dot(ea, ea), db = dot(eb, eb);
+    V3 ea = fma3(fma3(b, ta, c), ta, d), eb = fma3(fma3(b, tb, c), tb, d);
+    float da = dot_fma(ea, ea), db = dot_fma(eb, eb);
     bool use_b = db < da;
     t = use_b ? tb : ta;
     t_raw = use_b ? rb : ra;
-    s.z = z; s.m = m; s.n = n; s.sigma = use_b ? -1.f : 1.f;
+    s.sigma = use_b ? -1.f : 1.f;
   }
-  V3 e = d + (c + b * t) * t;
-  float dist = sqrtf(dot(e, e) + 1e-8f);
+  V3 e = fma3(fma3(b, t, c), t, d);
+  float dist = sqrtf(__fadd_rn(dot_fma(e, e), 1e-8f));
   s.t = t; s.t_raw = t_raw; s.e = e; s.dist = dist;
   float r1 = rec[R_QR1], r2 = rec[R_QR2];
-  return dist - (r1 + t * (r2 - r1));
+  return __fsub_rn(dist, fmaf(t, __fsub_rn(r2, r1), r1));
 }
 
 // Reverse mode of quad_eval for upstream w = dL/dSDF.
@@ -465,7 +458,7 @@ __device__ __forceinline__ V3 quad_adjoint(const float* rec, const QuadFwd& s, f
   } else if (gtr != 0.f) {
     // t_raw = sigma (m + n) z - kx, m = cos v, n = sqrt3 sin v, v = acos(q / (2 p z + 1e-8)) / 3,
     // z = sqrt(-p + 1e-8); p = ky - kx^2, q = kx (2 kx^2 - 3 ky) + kz
-    float gz = gtr * s.sigma * (s.m + s.n);
+    float gz = gtr * s.sigma * s.mn;
     const float gm = gtr * s.sigma * s.z;
     const float gn = gm;
     float sv, cv;
@@ -538,21 +531,19 @@ struct CubicFwd {
   V3 v;     // B(t) - pos
 };
 
-// INV (forwards): divisions by the segment's length squared as products with the record's
-// reciprocal. The backwards divide, for the same reason as quad_eval's.
+// INV (forwards): the pieces' reciprocal squared lengths from the record; the backwards, whose
+// registers are full, form the same values again.
 template <bool INV = true>
 __device__ __forceinline__ float cubic_eval(const float* rec, V3 pos, CubicFwd& s, bool power) {
   constexpr float step = 1.0f / CUBIC_SEGMENTS;
-  // Bound by issue, 10 pieces a pair: the reciprocal squared lengths come with the record
-  // (INV; else a fast division, 10 registers less, for the backward), the clamped parameter
-  // is formed again for the winner only (a NaN parameter, from a piece of length 0, clamps
-  // to 1, and a NaN distance never wins, as in the reference's loop). The distances keep
-  // the form pos - (s0 + ab t): where two pieces are nearly as close their rounding decides,
-  // and (pos - s0) - ab t, three instructions less, decided otherwise for a few samples
-  // (4e-4 of the control-point gradient's norm).
-  // 2000 mixed strokes, a quarter curves, 131,072 rays x 96, forward: 9.59 -> 8.22 ms with
-  // the quadratic's changes (quad_eval); 2000 curves, 16,411 rays x 64: forward 1.85 ->
-  // 1.65 ms, backward 1.74 -> 1.66.
+  // Bound by issue, 10 pieces a pair: the clamped parameter is formed again for the winner
+  // only (a NaN parameter, from a piece of length 0, clamps to 1, and a NaN distance never
+  // wins, as in the reference's loop). The distances keep the form pos - (s0 + ab t): where
+  // two pieces are nearly as close their rounding decides, and (pos - s0) - ab t, three
+  // instructions less, decided otherwise for a few samples (4e-4 of the control-point
+  // gradient's norm). Fusion is spelled out as in quad_eval. 2000 mixed strokes, a quarter
+  // curves, 131,072 rays x 96, forward: 9.59 -> 8.28 ms with the quadratic's form (quad_eval);
+  // 2000 curves, 16,411 rays x 64: forward 1.85 -> 1.64 ms, backward 1.74 -> 1.61.
   float best = 1e18f, tau_raw_best = 0.f;
   int seg = 0;
   float vtx[36], inv[CUBIC_SEGMENTS];
@@ -571,9 +562,9 @@ __device__ __forceinline__ float cubic_eval(const float* rec, V3 pos, CubicFwd& 
   for (int i = 1; i <= CUBIC_SEGMENTS; i++) {
     V3 s1 = v3(vtx[3 * i], vtx[3 * i + 1], vtx[3 * i + 2]);
     V3 ab = s1 - s0, w = pos - s0;
-    float tr = INV ? dot(w, ab) * inv[i - 1] : __fdividef(dot(w, ab), dot(ab, ab));
-    V3 dv = pos - (s0 + ab * clampf(tr, 0.f, 1.f));
-    float d2 = dot(dv, dv);
+    float tr = __fmul_rn(dot_fma(w, ab), INV ? inv[i - 1] : 1.f / dot_fma(ab, ab));
+    V3 dv = pos - fma3(ab, clampf(tr, 0.f, 1.f), s0);
+    float d2 = dot_fma(dv, dv);
     if (d2 < best) {
       best = d2;
       tau_raw_best = tr;
@@ -584,15 +575,16 @@ __device__ __forceinline__ float cubic_eval(const float* rec, V3 pos, CubicFwd& 
   const float tau_best = seg ? clampf(tau_raw_best, 0.f, 1.f) : 0.f;
   // the winning segment's t, as the reference's t_start (1 - tau) + t_end tau with
   // t_start = (seg - 1) step, t_end = seg step (the same float values as in its loop)
-  const float t_min = seg ? ((float)(seg - 1) * step) * (1.0f - tau_best) + ((float)seg * step) * tau_best : 0.f;
+  const float t_lo = __fmul_rn((float)(seg - 1), step), t_hi = __fmul_rn((float)seg, step);
+  const float t_min = seg ? fmaf(t_hi, tau_best, __fmul_rn(t_lo, __fsub_rn(1.0f, tau_best))) : 0.f;
   float w[4];
   curve_weights(t_min, w, power);
-  V3 P = xyz(cA) * w[0] + xyz(cB) * w[1] + xyz(cC) * w[2] + xyz(cD) * w[3];
+  V3 P = fma3(xyz(cD), w[3], fma3(xyz(cC), w[2], fma3(xyz(cA), w[0], xyz(cB) * w[1])));
   V3 v = P - pos;
-  float dist = sqrtf(dot(v, v));
+  float dist = sqrtf(dot_fma(v, v));
   s.t = t_min; s.tau = tau_best; s.tau_raw = tau_raw_best; s.seg = seg; s.v = v; s.dist = dist;
   float r1 = cA.w, r2 = cB.w;
-  return dist - (r1 + t_min * (r2 - r1));
+  return __fsub_rn(dist, fmaf(t_min, __fsub_rn(r2, r1), r1));
 }
 
 // Reverse mode of cubic_eval. compat != 0 reproduces the reference gradient

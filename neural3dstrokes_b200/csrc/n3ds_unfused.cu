@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(UF_WARPS * 32) uf_stroke_bwd_kernel(const UfSt
       sdf = compat ? prim_sdf(base, pl, rec) : prim_sdf_grad(base, pl, rec, &gsdf, gbp);
       if (kind & K_S3FAC) f = s3_factor(base, pl, xyz(rec4(rec)[R_S / 4]), rec);
     } else if (CLS == UF_QUAD) {
-      sdf = quad_eval<false>(rec, x, qf);
+      sdf = quad_eval(rec, x, qf);
     } else {
       sdf = cubic_eval<false>(rec, x, cf, base == B_CATMULL_ROM);
     }

@@ -281,3 +281,50 @@ def test_multi_pass_backward_matches_float64(cuda, n_samples, opaque):
     ref = oracle_grads(sc, rays, g_rgb, g_acc, torch.zeros(rays.n_rays), opaque=opaque)
     for name, leaf in zip(("x", "shape", "color", "density", "delta"), leaves):
         assert rel(leaf.grad, ref[name]) < GRAD_TOL, name
+
+
+@pytest.mark.parametrize("laplace", [True, False])
+@pytest.mark.parametrize("kind", ["ellipsoid", "quadratic_bezier", "cubic_bezier", "catmull_rom"])
+def test_strokes_behind_an_opaque_one_get_no_gradient(cuda, kind, laplace):
+    """The backward's prefixes repeat the forward's accumulations bit for bit, whatever is in
+    front: behind a hard stroke that covers every sample (alpha exactly 1) each suffix, and so
+    each gradient, is exactly zero. 40 strokes behind, 40 in front, several passes; without
+    culling, which may drop alphas below its threshold from the prefixes alone."""
+    g = torch.Generator().manual_seed(31)
+    n = 40
+    sc = scenes.make_strokes(["sphere"] * (n + 1) + [kind] * n, g)
+    sc.shape_params[n, :4] = torch.tensor([50.0, 0.0, 0.0, 0.0])
+    for cols in {"quadratic_bezier": (9, 10), "ellipsoid": ()}.get(kind, (12, 13)):
+        sc.shape_params[n + 1:, cols] += 0.2
+    rays = scenes.make_rays(60, 48, g)
+    delta = torch.full((2 * n + 1,), 0.1)
+    delta[n] = -1.0  # hard
+    sp = sc.shape_params.to(cuda).requires_grad_(True)
+    col, den = sc.color_params.to(cuda).requires_grad_(True), sc.density.to(cuda).requires_grad_(True)
+    rgb, acc, _ = render_strokes(rays.x.to(cuda), rays.radius.to(cuda), rays.tdist.to(cuda), rays.dirs.to(cuda), sp,
+                                 sc.sdf_ids.to(cuda), col, den, delta.to(cuda), laplace, True,
+                                 options=FieldOptions(cull_alpha=0.0, chunk_fwd=32, chunk_bwd=32))
+    up = torch.randn(60, 3, generator=g).to(cuda)
+    torch.autograd.backward([rgb, acc], [up, up[:, 0].contiguous()])
+    assert float(sp.grad[n + 1:].abs().max()) > 0.0 and bool(torch.isfinite(sp.grad[n + 1:]).all())
+    assert int(torch.count_nonzero(sp.grad[:n])) == 0
+    assert int(torch.count_nonzero(col.grad[:n])) == 0 and int(torch.count_nonzero(den.grad[:n])) == 0
+
+
+@pytest.mark.parametrize("schedule", SCHEDULES)
+@pytest.mark.parametrize("kind", ["quadratic_bezier", "cubic_bezier", "catmull_rom"])
+def test_linear_step_of_curves_matches_float64(cuda, kind, schedule):
+    """Gradients of curve strokes, and of primitives behind them, with the linear step, whose
+    adjoint divides by 1 - alpha (GRAD_TOL, normwise, as every gradient here)."""
+    g = torch.Generator().manual_seed(5)
+    sc = scenes.make_strokes(["sphere", "cube"] * 10 + [kind] * 20, g)
+    rays = scenes.make_rays(64, 40, g)
+    g_rgb, g_acc = torch.randn(64, 3, generator=g), torch.randn(64, generator=g)
+    chunk = 32 if schedule == "segments" else 0
+    (rgb, acc, _), leaves = run_field(sc, rays, cuda, delta=0.1, laplace=False, requires_grad=True,
+                                      opts=FieldOptions(schedule=schedule, chunk_fwd=chunk, chunk_bwd=chunk))
+    torch.autograd.backward([rgb, acc], [g_rgb.to(cuda), g_acc.to(cuda)])
+    ref = oracle_grads(sc, rays, g_rgb, g_acc, torch.zeros(64), delta=0.1, laplace=False)
+    assert rel(rgb, ref["rgb"]) < FWD_TOL and rel(acc, ref["acc"]) < FWD_TOL
+    for name, leaf in zip(("x", "shape", "color", "density", "delta"), leaves):
+        assert rel(leaf.grad, ref[name]) < GRAD_TOL, name
