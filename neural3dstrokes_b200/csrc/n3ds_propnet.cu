@@ -591,6 +591,16 @@ __device__ __forceinline__ void load_bwd_in(const NetLaunch& P, long long b, Bwd
   in.g = P.grad_density[b];
 }
 
+// A CTA that gave up: nothing of its tiles reaches the table either (the scatter follows
+// whatever happened here, and rows not written hold what the scratch held). Not inlined: the
+// layers' loop has no registers to spare.
+__device__ __noinline__ void clear_dfeat(float* dfeat, long long n, uint32_t stride) {
+  for (long long b = (long long)blockIdx.x * kTile + threadIdx.x; b < n; b += (long long)gridDim.x * kTile) {
+    float4* out = reinterpret_cast<float4*>(dfeat + b * stride);
+    for (uint32_t c = 0; c < stride / 4; c++) out[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+
 // CTAs per SM: 4 (the tensor-memory limit) with 8 feature columns; 16 hold more registers.
 constexpr int FP_CTAS(int features) { return features <= 8 ? 4 : 3; }
 // SCATTER: scatter the feature gradients into the table here; else write them to P.dfeat
@@ -786,6 +796,7 @@ __global__ void __launch_bounds__(kTile, SCATTER ? 3 : FP_CTAS(C * LMAX)) densit
     }
   }
   teardown(P, M, phase, timed_out, kColsBwd);
+  if (!SCATTER && timed_out) clear_dfeat(P.dfeat, P.n, P.stride);
 }
 
 // The table scatter of the split backward: the feature gradients of one point and chunk.

@@ -454,3 +454,29 @@ def test_split_network_matches_one_kernel(cuda, name, n):
     # float32 sums of n terms in two orders: sqrt(n) x 2^-24 relative to the largest sums
     for a, b in zip(*out):
         assert rel(a, b) < 4 * n ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("name", ["prop512_bbox", "error256_bbox"])
+def test_split_backward_that_gives_up_scatters_nothing(cuda, name):
+    """With the tensor-core work withheld (test hook) and a 50 us limit, the layers' kernel of
+    the split backward gives up on every tile (1000 tiles: more than resident CTAs): status
+    bit 2, and whatever the scratch held, the table gradient stays exactly zero."""
+    import ctypes
+    from neural3dstrokes_b200 import _lib
+    lib, net, n = _lib.load(), make_net(name, cuda), 128 * 999 + 5
+    x = ray_points(cuda, 2000, 64, 1.2)[:n].contiguous()
+    enc, lay = net.encoder, net.density_layer
+    params = [enc.embeddings, lay[0].weight, lay[0].bias, lay[2].weight, lay[2].bias]
+    status = torch.zeros(1, dtype=torch.int32, device=cuda)
+    s = mlp._net_struct(enc, *params[1:], net.density_bias, mlp._warp_mode(net.warp_fn, False), net.bbox_size, False,
+                        status=status, wait_limit_us=50, test_stall=True)
+    stride = lib.n3ds_density_net_feature_stride(enc.num_levels, enc.level_dim)
+    feats, g = torch.ones(n, stride, device=cuda), torch.ones(n, device=cuda)
+    grads = [torch.zeros_like(p) for p in params]
+    _lib.check(lib.n3ds_density_net_backward_scratch(
+        ctypes.byref(s), _lib.ptr(x), _lib.ptr(feats), _lib.ptr(g), n, *[_lib.ptr(t) for t in grads],
+        _lib.ptr(torch.full((n, stride), float("nan"), device=cuda)), _lib.stream_ptr()))
+    torch.cuda.synchronize(cuda)
+    assert int(status.item()) & 2
+    for t in grads:
+        assert int(torch.count_nonzero(t)) == 0
