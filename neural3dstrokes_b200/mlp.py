@@ -43,6 +43,14 @@ _SPLIT_BACKWARD = {1: (1 << 19, 1 << 24), 2: (1 << 16, 1 << 24), 4: (1 << 16, 1 
 HIDDEN = 64
 
 
+def _if_it_fits(make, *args, **kw):
+    """make(...), or None (the one-kernel form, which needs no such memory) without room."""
+    try:
+        return make(*args, **kw)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def _warp_mode(warp_fn, no_warp):
     if no_warp:
         return WARP_NONE
@@ -101,7 +109,10 @@ class _DensityNetFn(torch.autograd.Function):
         warped = torch.empty(n, 3, device=dev, dtype=torch.float32)
         # the record also carries the features from the encoding to the layers' kernel
         keep = need or _SPLIT_FORWARD[0] <= n <= _SPLIT_FORWARD[1]
-        feats = torch.empty(n, stride, device=dev, dtype=torch.float32) if keep else None
+        if need:
+            feats = torch.empty(n, stride, device=dev, dtype=torch.float32)
+        else:
+            feats = _if_it_fits(torch.empty, n, stride, device=dev, dtype=torch.float32) if keep else None
         net = _net_struct(enc, w1, b1, w2, b2, density_bias, warp, bbox_size, raw_output, **opts)
         with torch.cuda.device(dev):
             _lib.check(lib.n3ds_density_net_forward(ctypes.byref(net), _lib.ptr(x), n, _lib.ptr(density),
@@ -121,7 +132,7 @@ class _DensityNetFn(torch.autograd.Function):
         net = _net_struct(enc, w1, b1, w2, b2, density_bias, warp, bbox_size, raw_output, **opts)
         lib = _lib.load()
         lo, hi = _SPLIT_BACKWARD[embeddings.shape[1]]
-        scratch = torch.empty_like(feats) if lo <= x.shape[0] <= hi else None
+        scratch = _if_it_fits(torch.empty_like, feats) if lo <= x.shape[0] <= hi else None
         with torch.cuda.device(x.device):
             _lib.check(lib.n3ds_density_net_backward_scratch(
                 ctypes.byref(net), _lib.ptr(x), _lib.ptr(feats), _lib.ptr(g), x.shape[0],

@@ -480,3 +480,43 @@ def test_split_backward_that_gives_up_scatters_nothing(cuda, name):
     assert int(status.item()) & 2
     for t in grads:
         assert int(torch.count_nonzero(t)) == 0
+
+
+def _refuse_records(monkeypatch, refused):
+    """torch.empty / empty_like as they are, but out of memory for a shape in ``refused``."""
+    def wrap(make, shape_of):
+        def f(*a, **kw):
+            if shape_of(*a) in refused:
+                raise torch.OutOfMemoryError("refused by the test")
+            return make(*a, **kw)
+        return f
+    monkeypatch.setattr(torch, "empty", wrap(torch.empty, lambda *a: tuple(a)))
+    monkeypatch.setattr(torch, "empty_like", wrap(torch.empty_like, lambda t: tuple(t.shape)))
+
+
+def test_networks_run_without_memory_for_the_split_form(cuda, monkeypatch):
+    """The record of a forward that no backward follows and the backward's scratch are taken
+    for speed only: without memory for them the call runs as one kernel. Density bit-equal,
+    gradients to the rounding of sums in another order."""
+    net = make_net("prop512_bbox", cuda).requires_grad_(False)
+    x = ray_points(cuda, 512, 64, 1.2)
+    args = (net.encoder, net.density_layer, net.density_bias, net.warp_fn, net.bbox_size)
+    with torch.no_grad():
+        want, warped = mlp.density_net(x, *args)
+        with monkeypatch.context() as m:
+            _refuse_records(m, {(x.shape[0], 8)})
+            dens, w = mlp.density_net(x, *args)
+    assert torch.equal(dens, want) and torch.equal(w, warped)
+
+    net = make_net("error256_bbox", cuda)
+    x = ray_points(cuda, 1024, 64, 1.2)
+    g = torch.randn(x.shape[0], device=cuda, generator=torch.Generator(device=cuda).manual_seed(6))
+    d_w, _, grads_w = run_fused(net, x, g)
+    params = params_of(net)
+    d, _ = mlp.density_net(x, net.encoder, net.density_layer, net.density_bias, net.warp_fn, net.bbox_size)
+    with monkeypatch.context() as m:
+        _refuse_records(m, {(x.shape[0], 12)})
+        grads = torch.autograd.grad(d, params, g)
+    assert torch.equal(d.detach(), d_w)
+    for a, b in zip(grads, grads_w):
+        assert rel(a, b) < 4 * x.shape[0] ** 0.5 * 2.0 ** -24
