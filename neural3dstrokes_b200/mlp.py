@@ -35,11 +35,12 @@ from . import _lib
 from .gridencoder import GridEncoder
 
 WARP_SCALE, WARP_CONTRACT, WARP_NONE = 0, 1, 2
-# Points per call for which memory is taken so that the encoding and the table scatter run
-# as kernels of their own (where these are faster, n3ds_propnet.cu; at most 1 GB): a feature
-# record in a forward that no backward follows, a scratch for the feature gradients.
-_SPLIT_FORWARD = (1 << 15, 1 << 24)
-_SPLIT_BACKWARD = {1: (1 << 19, 1 << 24), 2: (1 << 16, 1 << 24), 4: (1 << 16, 1 << 24)}  # by channels
+# Points per call, by channels, for which memory is taken so that the encoding and the table
+# scatter run as kernels of their own (where these are faster, n3ds_propnet.cu, whose forward
+# splits from the same counts; at most 1 GB): a feature record in a forward that no backward
+# follows, a scratch for the feature gradients.
+_SPLIT_FORWARD = {1: (1 << 15, 1 << 24), 2: (1 << 18, 1 << 24), 4: (1 << 18, 1 << 24)}
+_SPLIT_BACKWARD = {1: (1 << 19, 1 << 24), 2: (1 << 16, 1 << 24), 4: (1 << 16, 1 << 24)}
 HIDDEN = 64
 
 
@@ -108,11 +109,11 @@ class _DensityNetFn(torch.autograd.Function):
         density = torch.empty(n, device=dev, dtype=torch.float32)
         warped = torch.empty(n, 3, device=dev, dtype=torch.float32)
         # the record also carries the features from the encoding to the layers' kernel
-        keep = need or _SPLIT_FORWARD[0] <= n <= _SPLIT_FORWARD[1]
+        lo, hi = _SPLIT_FORWARD.get(C, (1, 0))  # the library refuses other channel counts
         if need:
             feats = torch.empty(n, stride, device=dev, dtype=torch.float32)
         else:
-            feats = _if_it_fits(torch.empty, n, stride, device=dev, dtype=torch.float32) if keep else None
+            feats = _if_it_fits(torch.empty, n, stride, device=dev, dtype=torch.float32) if lo <= n <= hi else None
         net = _net_struct(enc, w1, b1, w2, b2, density_bias, warp, bbox_size, raw_output, **opts)
         with torch.cuda.device(dev):
             _lib.check(lib.n3ds_density_net_forward(ctypes.byref(net), _lib.ptr(x), n, _lib.ptr(density),

@@ -520,3 +520,23 @@ def test_networks_run_without_memory_for_the_split_form(cuda, monkeypatch):
     assert torch.equal(d.detach(), d_w)
     for a, b in zip(grads, grads_w):
         assert rel(a, b) < 4 * x.shape[0] ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("name,n,split", [("prop512_bbox", 32767, False), ("prop512_bbox", 32768, True),
+                                          ("error256_bbox", 262143, False), ("error256_bbox", 262144, True),
+                                          ("c4_contract", 262143, False), ("c4_contract", 262144, True)])
+def test_record_taken_only_where_the_forward_splits(cuda, name, n, split):
+    """A forward that no backward follows allocates a feature record only where the native
+    dispatch reads it (from 2^15 points at one channel, 2^18 at more)."""
+    net = make_net(name, cuda).requires_grad_(False)
+    x = ray_points(cuda, (n + 63) // 64, 64, 1.2)[:n].contiguous()
+    args = (net.encoder, net.density_layer, net.density_bias, net.warp_fn, net.bbox_size)
+    with torch.no_grad():
+        torch.cuda.synchronize(cuda)
+        torch.cuda.reset_peak_memory_stats(cuda)
+        base = torch.cuda.memory_stats(cuda)["requested_bytes.all.current"]
+        out = mlp.density_net(x, *args)
+        peak = torch.cuda.memory_stats(cuda)["requested_bytes.all.peak"] - base
+    # outputs: 16 bytes a point; the record: 32 to 48 more
+    assert (peak >= 48 * n) == split, (peak, n)
+    del out
