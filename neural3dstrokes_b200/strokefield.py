@@ -93,8 +93,13 @@ def annealed_delta(field, window):
 
 def _plain_state(field, coords, dev):
     """The module's state is what the one-launch form reads: an int32 count and float32
-    densities on the coordinates' device, host numbers for the settings."""
+    densities on the coordinates' device, host numbers for the settings, counts that its int32
+    fields hold (others: the tensor expressions, which refuse them or compute in float64)."""
     step, den = field.stroke_step, field.density_params
+    limit = getattr(field, "stroke_step_limit", None)
+    if not all(-2**31 <= v < 2**31 for v in (field.max_opt_strokes, field.max_num_strokes, limit or 0)) or \
+            int(field.max_num_strokes) != field.max_num_strokes:
+        return False
     return (torch.is_tensor(step) and step.is_cuda and step.device == dev and step.dtype == torch.int32 and
             step.numel() == 1 and den.is_cuda and den.device == dev and den.dtype == torch.float32 and
             coords.dtype == torch.float32 and

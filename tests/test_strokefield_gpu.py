@@ -281,3 +281,24 @@ def test_module_inputs_match_the_tensor_expressions(cuda, n, step, limit, traini
     f.stroke_step = f.stroke_step.to(torch.int64)  # the torch expressions
     for a, b in zip(ours, f.render(x, radius, tdist, dirs)):
         assert torch.equal(a, b)
+
+
+def test_module_counts_beyond_the_one_launch_form(cuda):
+    """Counts that the one-launch form's int32 cannot hold keep the tensor expressions: a
+    step limit of 2^40 is refused as torch refuses it, a field size of 2^33 (or of infinity)
+    anneals by it."""
+    f = make_field("ellipsoid", 52, True, cuda)
+    coords, radius, tdist, dirs = rays_for(cuda)
+    want = f.render(coords, radius, tdist, dirs)
+    f.stroke_step_limit = 2 ** 40
+    with pytest.raises(RuntimeError):
+        f.render(coords, radius, tdist, dirs)
+    f.stroke_step_limit = None
+    f.max_num_strokes = 2 ** 33
+    got = f.render(coords, radius, tdist, dirs)
+    f.max_num_strokes = float("inf")
+    assert torch.equal(f.render(coords, radius, tdist, dirs)[0], got[0])
+    f.max_num_strokes, f.sdf_delta_eval = MAX, f.sdf_delta  # annealed by 52 / 2^33: sdf_delta
+    for a, b in zip(got, f.render(coords, radius, tdist, dirs)):
+        assert rel(a, b) < FWD_TOL
+    assert not torch.equal(got[0], want[0])
