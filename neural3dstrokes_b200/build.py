@@ -29,7 +29,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # several instructions each; the 1-2 ulp difference is far inside the 1e-5 tolerance.
 FAST_MATH = ["-prec-sqrt=false", "-prec-div=false", "-ftz=true"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", INCLUDE, "-I", CSRC] + \
-    ([] if os.environ.get("N3DS_IEEE_MATH") else FAST_MATH)
+    (["-DN3DS_IEEE_MATH"] if os.environ.get("N3DS_IEEE_MATH") else FAST_MATH)
 
 
 def nvcc_path():

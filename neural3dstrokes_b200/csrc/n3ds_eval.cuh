@@ -82,10 +82,10 @@ __device__ __forceinline__ float pair_alpha_common(const float* rec, V3 x, float
 
 // dL/dm of the soft step given G = (1 - alpha) dL/dalpha (division-safe form).
 __device__ __forceinline__ float soft_dm_from_G(int mode, float m, float alpha, float G) {
-  if (mode == STEP_LAPLACE) return m <= 0.f ? __fdividef(G * alpha, 1.f - alpha) : G;
+  if (mode == STEP_LAPLACE) return m <= 0.f ? fast_div(G * alpha, 1.f - alpha) : G;
   if (mode == STEP_LINEAR) {
     float a = m + 0.5f;
-    return (a > 0.f && a < 0.9999f) ? __fdividef(G, 1.f - alpha) : 0.f;
+    return (a > 0.f && a < 0.9999f) ? fast_div(G, 1.f - alpha) : 0.f;
   }
   return 0.f;
 }

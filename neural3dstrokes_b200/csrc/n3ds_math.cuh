@@ -28,6 +28,15 @@ __host__ __device__ __forceinline__ V3 operator-(float s, V3 a) { return {s - a.
 __host__ __device__ __forceinline__ V3& operator+=(V3& a, V3 b) { a.x += b.x; a.y += b.y; a.z += b.z; return a; }
 __host__ __device__ __forceinline__ V3& operator-=(V3& a, V3 b) { a.x -= b.x; a.y -= b.y; a.z -= b.z; return a; }
 __host__ __device__ __forceinline__ float dot(V3 a, V3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// A division whose last places do not matter: the build's approximate division without its
+// range check; the rounded one in an IEEE build.
+__device__ __forceinline__ float fast_div(float a, float b) {
+#ifdef N3DS_IEEE_MATH
+  return __fdiv_rn(a, b);
+#else
+  return __fdividef(a, b);
+#endif
+}
 // dot and a s + c with the fusion spelled out: the same bits in every kernel, where the
 // plain expressions leave the choice of the fused product to each kernel's compilation.
 __device__ __forceinline__ float dot_fma(V3 a, V3 b) { return fmaf(a.z, b.z, fmaf(a.x, b.x, __fmul_rn(a.y, b.y))); }

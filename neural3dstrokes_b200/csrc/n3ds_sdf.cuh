@@ -321,7 +321,7 @@ __device__ __forceinline__ float quad_newton(float s, float pt, float q) {
   for (int it = 0; it < 2; it++) {
     const float g = fmaf(fmaf(s, s, __fmul_rn(3.f, pt)), s, q);
     const float gd = __fmul_rn(3.f, fmaf(s, s, pt));
-    if (fabsf(gd) > 1e-12f) s = __fsub_rn(s, __fdividef(g, gd));
+    if (fabsf(gd) > 1e-12f) s = __fsub_rn(s, fast_div(g, gd));
   }
   return s;
 }
@@ -369,7 +369,7 @@ __device__ __forceinline__ float quad_eval(const float* rec, V3 pos, QuadFwd& s)
     s.pos_branch = 1;
     const float H = sqrtf(__fadd_rn(h, 1e-8f));
     const float u = copysignf(cbrtf(__fadd_rn(fabsf(q), H) * 0.5f), -q);
-    s0 = __fsub_rn(u, __fdividef(pt, u));
+    s0 = __fsub_rn(u, fast_div(pt, u));
   } else {
     s.pos_branch = 0;
     z = sqrtf(__fadd_rn(-p, 1e-8f));

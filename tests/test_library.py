@@ -3,6 +3,10 @@
 import ctypes
 import os
 import re
+import subprocess
+import sys
+
+import pytest
 
 from neural3dstrokes_b200 import _lib
 
@@ -50,3 +54,23 @@ def test_pure_host_calls():
     rc = lib.n3ds_stroke_forward(None, None, None, None, 0, None, None, None, None, None, 10, 1, 4, 4, 3, 0xC0, 0,
                                  0.02, 1, 1, None, 0, None)
     assert rc in (1, 2)  # sdf base 12 does not exist
+
+
+@pytest.mark.parametrize("ieee", [False, True])
+def test_ieee_build_has_no_approximate_division(ieee):
+    """Under N3DS_IEEE_MATH every division of the kernels is rounded: after preprocessing with
+    that build's flags no source line of csrc calls the approximate one. (The default build
+    does, in one place.)"""
+    env = dict(os.environ, N3DS_IEEE_MATH="1" if ieee else "")
+    flags = subprocess.run([sys.executable, "-c", "from neural3dstrokes_b200 import build as b; print(b.nvcc_path(), *b.FLAGS)"],
+                           cwd=ROOT, env=env, capture_output=True, text=True, check=True).stdout.split()
+    calls, own = 0, False
+    src = os.path.join(ROOT, "neural3dstrokes_b200", "csrc", "n3ds_field.cu")
+    out = subprocess.run(flags + ["-E", src], capture_output=True, text=True, check=True).stdout
+    for line in out.splitlines():
+        mark = re.match(r'# \d+ "(.*)"', line) or re.match(r'#line \d+ "(.*)"', line)
+        if mark:
+            own = "csrc" in mark.group(1)
+        elif own:
+            calls += line.count("__fdividef(")
+    assert calls == (0 if ieee else 1)
