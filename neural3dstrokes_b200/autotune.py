@@ -5,11 +5,11 @@ on its own data for each candidate launch configuration and keeps the fastest:
 
 * work decomposition (``schedule``): 32-sample segments with every lane evaluating
   each surviving stroke, or 64-sample units with packed (sample, stroke) pairs;
-* warps per CTA (rays in flight per SM), forward and backward separately (the
-  segment kernels fit 32 warps; the backward's 32-warp build is held to 64 registers
-  and spills a little: on config 3 its backward alone measured 5.12 against 5.27 ms
-  and a whole tuned step within noise of 24 warps, on Bezier tubes (config 2) 26.2
-  against 25.1 ms, so the tuner decides per workload; the run kernels 16);
+* warps per CTA (rays in flight per SM), forward and backward separately (the segment
+  kernels run up to 32; the backward's 28-warp build, 72 registers, is the default and was
+  the fastest on every workload measured, 24 / 28 / 32 warps, backward alone: 16 mixed
+  scenes 4.27 / 4.13 / 4.42 ms, Bezier tubes (config 2) 19.3 / 18.9 / 19.4, 500 primitives
+  1.31 / 1.25 / 1.33; the run kernels 16);
 * strokes per shared-memory stage: the largest that fits, or half of it (more passes,
   less shared memory per CTA);
 * samples per warp claim (segment schedule): a warp takes 1, 2 or 4 rays (64, 128 or
@@ -52,8 +52,8 @@ def candidates(grad_mode: str = "exact", cull_alpha: float = 1e-9, forward_only:
     out = []
     # (schedule, forward warps, backward warps): up to 32 warps per CTA for the
     # segment kernels, 16 for the run kernels
-    shapes = [("segments", 32, 32), ("segments", 32, 24), ("segments", 32, 20), ("segments", 24, 16),
-              ("segments", 16, 16), ("runs", 16, 16)]
+    shapes = [("segments", 32, 32), ("segments", 32, 28), ("segments", 32, 24), ("segments", 32, 20),
+              ("segments", 24, 16), ("segments", 16, 16), ("runs", 16, 16)]
     for schedule, wf, wb in shapes:
         for half in (False, True):
             # chunk 0 = the largest stage that fits; the halved stage (-1) is resolved later

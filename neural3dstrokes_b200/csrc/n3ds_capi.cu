@@ -99,7 +99,7 @@ WsLayout ws_layout(long long total_rays, int N, long long S, long long n_mask_wo
 struct Resolved {
   float cull_m, cull_alpha;
   int chunk_fwd, chunk_bwd, warps, schedule, grad_mode;
-  int warps_fwd, warps_bwd;  // per direction (the forward segment kernel runs 24 warps by default)
+  int warps_fwd, warps_bwd;  // per direction (the segment kernels run 32 and 28 by default)
   void* const* events;
   int forward_only;
   int count_pairs;
@@ -135,9 +135,11 @@ Resolved resolve(const n3ds_options_t* o) {
     return best;
   };
   // defaults: the fastest measured on the benchmark workloads. Segment backward: 28 warps
-  // (72 registers, 16 bytes of spill), seven per scheduler against the exposed latency of
-  // record loads and shuffles; 32 would spill 60 bytes in the stroke loop (16 uneven
-  // mixed scenes: 24 warps 4.34 ms, 28 4.16, 32 4.48; 2000 curves 1.73 / 1.75 / 1.76)
+  // (72 registers, 16 bytes of spill at most), seven per scheduler against the exposed latency of
+  // record loads and shuffles; 32 spill 36 to 52 in the stroke loop. Backward alone,
+  // 24 / 28 / 32 warps in turn: 16 uneven mixed scenes 4.27 / 4.13 / 4.42 ms, 500 primitives
+  // 1.31 / 1.25 / 1.33, 2000 ellipsoids 1.69 / 1.64 / 1.74, primitives and curves 1.27 / 1.24
+  // / 1.33, 2000 curves 1.69 / 1.66 / 1.68, 500 curves 1.40 / 1.35 / 1.35: one rule for all.
   const int wf = o->warps > 0 ? o->warps : (runs ? 16 : 32);
   const int wb = o->warps_bwd > 0 ? o->warps_bwd : (runs ? 16 : 28);
   r.warps_fwd = runs ? pick(wf, {4, 8, 16}) : pick(wf, {4, 8, 16, 24, 32});

@@ -477,7 +477,8 @@ __device__ __forceinline__ void compose_skip(const float* rec, float a, CompAdj&
 // 300 warp instructions per segment and kept stroke, a fifth of them the 16-slot
 // reduction). 16 uneven mixed scenes, 347k rays x 64 samples: 4.77 ms at 24 warps; 4.34
 // with SDF and gradient in one type switch, the one scale cancelled in the torque, g_T
-// T_final formed once per segment and a fast division; 4.16 at 28 warps (72 registers).
+// T_final formed once per segment and a fast division; 4.16 at 28 warps (72 registers),
+// 4.13 with the curves' one form of evaluation.
 template <int WARPS, bool GX, int COMPAT, bool MASKS, bool STATS>
 __global__ void __launch_bounds__(WARPS * 32, 1) seg_bwd_kernel(const __grid_constant__ SegLaunch L) {
   extern __shared__ __align__(128) unsigned char smem[];

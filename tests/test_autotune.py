@@ -102,3 +102,15 @@ def test_tuning_keeps_results(cuda):
     field.forward()
     torch.cuda.synchronize()
     assert rel(field.rgb, ref) < FWD_TOL
+
+
+@pytest.mark.parametrize("schedule", ["segments", "runs"])
+def test_candidate_set_holds_the_default_launch(schedule):
+    """The warps that a field runs untuned are among those that the tuner tries."""
+    import ctypes
+    from neural3dstrokes_b200 import _lib
+    out = _lib.Options()
+    _lib.check(_lib.load().n3ds_field_resolve_options(ctypes.byref(FieldOptions(schedule=schedule).c()),
+                                                      ctypes.byref(out)))
+    tried = {(o.warps, o.warps_bwd) for o in autotune.candidates() if o.schedule == schedule}
+    assert (int(out.warps), int(out.warps_bwd)) in tried
