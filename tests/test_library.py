@@ -74,3 +74,16 @@ def test_ieee_build_has_no_approximate_division(ieee):
         elif own:
             calls += line.count("__fdividef(")
     assert calls == (0 if ieee else 1)
+
+
+def test_build_without_reference_sources(tmp_path, monkeypatch):
+    """build() compiles the comparators only where the reference's sources are: an empty
+    checkout folder is as good as none."""
+    import __graft_entry__ as entry
+    from neural3dstrokes_b200 import build as nb
+    from oracle import build_ref
+    monkeypatch.setattr(nb, "build", lambda *a, **k: _lib.load()._name)
+    monkeypatch.setattr(build_ref, "reference_root", lambda: str(tmp_path))
+    monkeypatch.setattr(build_ref, "built_path", lambda: None)
+    monkeypatch.setattr(build_ref, "grid_built_path", lambda: None)
+    entry.build()
