@@ -540,3 +540,41 @@ def test_record_taken_only_where_the_forward_splits(cuda, name, n, split):
     # outputs: 16 bytes a point; the record: 32 to 48 more
     assert (peak >= 48 * n) == split, (peak, n)
     del out
+
+
+@pytest.mark.parametrize("name,n", [("prop512_bbox", 32768), ("prop2048_contract", 32768 + 77),
+                                    ("error256_bbox", 262144 + 1), ("c4_contract", 262144 + 129)])
+def test_split_network_warps_and_nan_points(cuda, name, n):
+    """Where the forward splits, its warped coordinates equal the one-kernel form's bit for
+    bit, NaN and out-of-grid points included; and with NaN points in the backward the split
+    form's gradients are NaN where the one-kernel form's are and agree elsewhere."""
+    import ctypes
+    from neural3dstrokes_b200 import _lib
+    lib, net = _lib.load(), make_net(name, cuda)
+    x = ray_points(cuda, (n + 63) // 64, 64, 1.6 if net.warp_fn is None else 3.0)[:n].contiguous()
+    x[5], x[n - 1, 1] = float("nan"), float("nan")
+    enc, lay = net.encoder, net.density_layer
+    params = [enc.embeddings, lay[0].weight, lay[0].bias, lay[2].weight, lay[2].bias]
+    s = mlp._net_struct(enc, *params[1:], net.density_bias, mlp._warp_mode(net.warp_fn, False), net.bbox_size, False)
+    stride = lib.n3ds_density_net_feature_stride(enc.num_levels, enc.level_dim)
+    feats = torch.empty(n, stride, device=cuda)
+    res = []
+    for rec in (feats, None):
+        dens, warped = torch.full((n,), -1.0, device=cuda), torch.full((n, 3), -7.0, device=cuda)
+        _lib.check(lib.n3ds_density_net_forward(ctypes.byref(s), _lib.ptr(x), n, _lib.ptr(dens), _lib.ptr(rec),
+                                                _lib.ptr(warped), _lib.stream_ptr()))
+        res.append((dens, warped))
+    for a, b in zip(*res):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(), b.nan_to_num())
+    assert bool(res[0][1][5].isnan().all()) and bool(res[0][1][n - 1].isnan().any())
+    g = torch.randn(n, device=cuda, generator=torch.Generator(device=cuda).manual_seed(4))
+    out = []
+    for scratch in (None, torch.full((n, stride), float("nan"), device=cuda)):
+        grads = [torch.zeros_like(p) for p in params]
+        _lib.check(lib.n3ds_density_net_backward_scratch(
+            ctypes.byref(s), _lib.ptr(x), _lib.ptr(feats), _lib.ptr(g), n, *[_lib.ptr(t) for t in grads],
+            _lib.ptr(scratch), _lib.stream_ptr()))
+        out.append(grads)
+    for a, b in zip(*out):
+        assert torch.equal(a.isnan(), b.isnan())
+        assert rel(a.nan_to_num(), b.nan_to_num()) < 4 * n ** 0.5 * 2.0 ** -24

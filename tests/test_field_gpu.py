@@ -328,3 +328,27 @@ def test_linear_step_of_curves_matches_float64(cuda, kind, schedule):
     assert rel(rgb, ref["rgb"]) < FWD_TOL and rel(acc, ref["acc"]) < FWD_TOL
     for name, leaf in zip(("x", "shape", "color", "density", "delta"), leaves):
         assert rel(leaf.grad, ref[name]) < GRAD_TOL, name
+
+
+@pytest.mark.parametrize("laplace", [True, False])
+@pytest.mark.parametrize("kind", [k for k in scenes.EVERY_KIND if k not in ("ellipsoid", "quadratic_bezier",
+                                                                           "cubic_bezier", "catmull_rom")])
+def test_primitives_in_front_of_an_opaque_stroke_leave_no_residue(cuda, kind, laplace):
+    """As test_strokes_behind_an_opaque_one_get_no_gradient, for every other shape in front."""
+    g = torch.Generator().manual_seed(37)
+    n = 40
+    sc = scenes.make_strokes(["sphere"] * (n + 1) + [kind] * n, g)
+    sc.shape_params[n, :4] = torch.tensor([50.0, 0.0, 0.0, 0.0])
+    rays = scenes.make_rays(60, 48, g)
+    delta = torch.full((2 * n + 1,), 0.1)
+    delta[n] = -1.0  # hard
+    sp = sc.shape_params.to(cuda).requires_grad_(True)
+    col, den = sc.color_params.to(cuda).requires_grad_(True), sc.density.to(cuda).requires_grad_(True)
+    rgb, acc, _ = render_strokes(rays.x.to(cuda), rays.radius.to(cuda), rays.tdist.to(cuda), rays.dirs.to(cuda), sp,
+                                 sc.sdf_ids.to(cuda), col, den, delta.to(cuda), laplace, True,
+                                 options=FieldOptions(cull_alpha=0.0, chunk_fwd=32, chunk_bwd=32))
+    up = torch.randn(60, 3, generator=g).to(cuda)
+    torch.autograd.backward([rgb, acc], [up, up[:, 0].contiguous()])
+    assert float(sp.grad[n + 1:].abs().max()) > 0.0
+    assert int(torch.count_nonzero(sp.grad[:n])) == 0
+    assert int(torch.count_nonzero(col.grad[:n])) == 0 and int(torch.count_nonzero(den.grad[:n])) == 0

@@ -395,3 +395,32 @@ def test_level_rows_transposition_is_exact(cuda, monkeypatch, B, L, C, dtype):
     rows = ge._rows_of_levels(t, B, L, C)
     assert rows.is_contiguous() and torch.equal(rows, t.permute(1, 0, 2).reshape(B, L * C))
     assert torch.equal(ge._levels_of_rows(rows, B, L, C), t)
+
+
+@pytest.mark.parametrize("C,L,B,tiled", [(4, 4, (1 << 19) - 1, False), (4, 4, 1 << 19, True), (2, 16, 1 << 18, True),
+                                         (1, 16, 1 << 19, False)])
+def test_encoder_at_the_transposition_threshold(cuda, C, L, B, tiled):
+    """The module on both sides of the size from which rows are transposed by the kernel (32 MB,
+    elements of at least 8 bytes): features bit-equal to torch's permutation of the level-major
+    outputs, table gradients to the order of the atomics (8 B / 729 terms a row at the coarsest
+    level: 4 sqrt(terms) 2^-24)."""
+    enc = ge.GridEncoder(input_dim=3, num_levels=L, level_dim=C, base_resolution=8, per_level_scale=1.1,
+                         log2_hashmap_size=13).to(cuda)
+    g = torch.Generator(device=cuda).manual_seed(C)
+    with torch.no_grad():
+        enc.embeddings.uniform_(-1, 1, generator=g)
+    x = torch.rand(B, 3, device=cuda, generator=g)
+    assert ge._tiled(torch.empty(L, B, C, device=cuda), B, L, C * 4) == tiled
+    y = ge.grid_encode(x, enc.embeddings, enc.offsets, enc.per_level_scale, enc.base_resolution, False, enc.gridtype_id,
+                       enc.align_corners, enc.interp_id)
+    S, H = float(np.log2(enc.per_level_scale)), enc.base_resolution
+    lv = torch.empty(L, B, C, device=cuda)
+    common = (B, 3, C, L, S, H, None, enc.gridtype_id, enc.align_corners, enc.interp_id)
+    ge.grid_encode_forward(x, enc.embeddings.detach(), enc.offsets, lv, *common)
+    assert torch.equal(y.detach(), lv.permute(1, 0, 2).reshape(B, L * C))
+    up = torch.randn(B, L * C, device=cuda, generator=g)
+    got, = torch.autograd.grad(y, enc.embeddings, up)
+    want = torch.zeros_like(enc.embeddings)
+    ge.grid_encode_backward(up.view(B, L, C).permute(1, 0, 2).contiguous(), x, enc.embeddings.detach(), enc.offsets,
+                            want, B, 3, C, L, S, H, None, None, enc.gridtype_id, enc.align_corners, enc.interp_id)
+    assert rel(got, want) < 4 * (8 * B / 729) ** 0.5 * 2.0 ** -24

@@ -352,3 +352,44 @@ def test_stroke_op_gradients_ignore_what_buffers_held(cuda, monkeypatch, shape, 
                        scenes.SDF_ID[shape], 3 if color == "constant_sh3" else 0, 0.1, True, True)
     for a, b in zip(got, (want[2], want[0], want[1])):
         assert rel(a, b) < GRAD_TOL
+
+
+@pytest.mark.parametrize("mode", ["exact", "compat"])
+@pytest.mark.parametrize("shape,color,P,S", [("cube", "constant_rgb", 64, 33), ("obb", "gradient_rgb", 200, 130),
+                                             ("cubic_bezier", "gradient_rgb", 65, 32),
+                                             ("quadratic_bezier", "constant_sh2", 64, 31)])
+def test_written_stroke_gradients_in_both_modes(cuda, monkeypatch, mode, shape, color, P, S):
+    """The writing backward against the accumulating one on cleared buffers, in both gradient
+    modes and with the position gradients of gradient rgb, every buffer that the call
+    allocates (the workspace too) filled with NaN (GRAD_TOL, normwise)."""
+    from neural3dstrokes_b200 import strokes as st_api
+    g = torch.Generator().manual_seed(P + S)
+    fn, n, dim = st_api.get_stroke(shape, color, "recon")[:3]
+    prm = scenes.make_strokes([shape] * S, g).shape_params[:, :n].contiguous().to(cuda)
+    col = torch.rand(S, dim, generator=g).to(cuda)
+    x, r = (torch.rand(P, 3, generator=g) * 2 - 1).to(cuda), torch.ones(P, device=cuda)
+    vd = torch.nn.functional.normalize(torch.randn(P, 3, generator=g), dim=-1).to(cuda)
+    ga, gc = torch.randn(P, S, generator=g).to(cuda), torch.randn(P, S, 3, generator=g).to(cuda)
+    leaves = [t.requires_grad_(True) for t in (x, prm, col)]
+    alpha, c, _, _ = fn(x, r, vd, prm, col, 0.1, True, True)
+
+    def poisoned(make):
+        def f(*a, **kw):
+            t = make(*a, **kw)
+            return t.fill_(255) if t.dtype == torch.uint8 else t.fill_(float("nan"))
+        return f
+
+    sl.set_grad_mode(mode)
+    try:
+        with monkeypatch.context() as m:
+            m.setattr(torch, "empty", poisoned(torch.empty))
+            m.setattr(torch, "empty_like", poisoned(torch.empty_like))
+            got = torch.autograd.grad((alpha, c), leaves, (ga, gc))
+        want = [torch.zeros_like(t) for t in (prm, col, x)]
+        sl.stroke_backward(*want, ga, gc, torch.empty(0, device=cuda), x.detach(), r, vd, alpha.detach(), prm.detach(),
+                           col.detach(), scenes.SDF_ID[shape],
+                           {"constant_rgb": 0, "gradient_rgb": 1, "constant_sh2": 2}[color], 0.1, True, True)
+    finally:
+        sl.set_grad_mode("exact")
+    for a, b in zip(got, (want[2], want[0], want[1])):
+        assert rel(a, b) < GRAD_TOL
