@@ -91,14 +91,16 @@ def annealed_delta(field, window):
     return d.to(torch.float32)
 
 
+_I32 = 2**31
+
+
 def _plain_state(field, coords, dev):
     """The module's state is what the one-launch form reads: an int32 count and float32
     densities on the coordinates' device, host numbers for the settings, counts that its int32
     fields hold (others: the tensor expressions, which refuse them or compute in float64)."""
     step, den = field.stroke_step, field.density_params
-    limit = getattr(field, "stroke_step_limit", None)
-    if not all(-2**31 <= v < 2**31 for v in (field.max_opt_strokes, field.max_num_strokes, limit or 0)) or \
-            int(field.max_num_strokes) != field.max_num_strokes:
+    opt, num, limit = field.max_opt_strokes, field.max_num_strokes, getattr(field, "stroke_step_limit", None) or 0
+    if not (-_I32 <= opt < _I32 and -_I32 <= num < _I32 and -_I32 <= limit < _I32 and int(num) == num):
         return False
     return (torch.is_tensor(step) and step.is_cuda and step.device == dev and step.dtype == torch.int32 and
             step.numel() == 1 and den.is_cuda and den.device == dev and den.dtype == torch.float32 and
