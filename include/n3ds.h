@@ -518,7 +518,7 @@ int n3ds_grid_encode_backward(const void* grad, const float* inputs, const void*
                               uint32_t H, const void* dy_dx, void* grad_inputs, uint32_t gridtype,
                               int32_t align_corners, uint32_t interpolation, int32_t dtype, n3ds_stream_t stream);
 /* The encoder's [L, B, C] tensors to rows [B, L, C] (to_rows nonzero) or back; unit_bytes
- * = C * element size (2 to 64), L * unit_bytes at most 40 KB. src and dst aligned to the
+ * = C * element size (2 to 64), L * unit_bytes at most 40 KB - 16. src and dst aligned to the
  * unit (16 bytes at most). */
 int n3ds_grid_transpose(const void* src, void* dst, uint32_t B, uint32_t L, uint32_t unit_bytes, int32_t to_rows,
                         n3ds_stream_t stream);

@@ -187,9 +187,11 @@ __global__ void __launch_bounds__(COL_WARPS * 32) uf_gradient_rgb_bwd_kernel(con
 // one view direction at a time, evaluates the field once and streams the colour rows. A row
 // of the 32-stroke block is 96 consecutive floats: element lane + 32 k of it belongs to
 // stroke e / 3, channel e % 3, so three coalesced accesses move it; the backward sums
-// the upstream rows by element and takes its own stroke's sums once per piece. HBM bound
-// (12 B per pair): 19,904 samples x 131 strokes, SH3: forward 19 -> 9 us, backward 115
-// -> 36 us (the harmonics, sigmoid and 27 parameter gradients per sample and stroke before).
+// the upstream rows by element and takes its own stroke's sums once per piece. 12 B per pair,
+// 31 MB at 19,904 samples x 131 strokes, SH3, most of it in L2: the forward is bound by its
+// stores (19 -> 9 us, 3.5 TB/s), the backward, at 117 registers, by the latency of the row
+// loads and the parameter atomics (115 -> 36 us, 0.9 TB/s, issue 11 %). Before, each sample and
+// stroke formed the harmonics, the sigmoid and 27 parameter gradients.
 constexpr int SH_PIECE = 16;
 
 __device__ __forceinline__ float sel3(int q, float a, float b, float c) { return q == 0 ? a : (q == 1 ? b : c); }

@@ -271,9 +271,10 @@ __global__ void dilate_kernel(const DilateArgs A) {
 
 // Sample positions and radii of a proposal level (cast_rays, render.py:20-25): t = (t0 + t1)
 // / 2, x = d t + o, radius = r t, each operation rounded. A warp per ray, a lane per
-// coordinate, stores coalesced. HBM bound (16 B written per sample): 16,384 rays x 64 in
-// 8 us, 48 us as five torch operations over broadcast operands (22 with a thread per
-// coordinate of the whole level, whose 64-bit divisions took the time).
+// coordinate, stores coalesced. Bound by the latency of a warp's first loads and by issue
+// (63 % of the slots): 16,384 rays x 64, 21 MB that stay in L2, in 8 us, 2.6 TB/s; 48 us as
+// five torch operations over broadcast operands (22 with a thread per coordinate of the
+// whole level, whose 64-bit divisions took the time).
 __global__ void __launch_bounds__(256) ray_points_kernel(float* coords, float* radius, const float* tdist,
                                                          const float* origins, const float* dirs, const float* radii,
                                                          long long R, int N) {
@@ -293,8 +294,9 @@ __global__ void __launch_bounds__(256) ray_points_kernel(float* coords, float* r
 }
 
 // compute_alpha_weights' weights (render.py:29-48) of one level, a warp per ray:
-// alpha = 1 - exp(-sigma dt |d|), trans = exp(-sum of the optical depths before). HBM bound
-// (8 B per sample): 16,384 rays x 64 in 7 us, 30 us as nine torch operations.
+// alpha = 1 - exp(-sigma dt |d|), trans = exp(-sum of the optical depths before). Bound by the
+// latency of a warp's loads and by issue (59 % of the slots), 12 B per sample: 16,384 rays x
+// 64 in 7 us, 1.8 TB/s; 30 us as nine torch operations.
 __global__ void __launch_bounds__(256) ray_weights_kernel(float* weights, const float* density, const float* tdist,
                                                           const float* dirs, long long R, int N, int opaque) {
   const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
